@@ -80,8 +80,9 @@ struct kc_batch {
     struct Lists {
         int cap_tests = 0, cap_rows = 0, cap_cols = 0;
         TestDesc *d_desc = nullptr, *h_desc = nullptr;
-        WorkItem *d_rows = nullptr, *h_rows = nullptr, *d_cols = nullptr, *h_cols = nullptr;
-        int *d_cnt = nullptr, *h_cnt = nullptr;
+        WorkItem *d_rows = nullptr, *h_rows = nullptr;
+        WorkItem *d_cols = nullptr, *h_cols = nullptr;  // second half: groups of 4 columns
+        int *d_cnt = nullptr, *h_cnt = nullptr;  // items: rows, columns, groups of 4 columns
         unsigned *d_flow = nullptr;  // control words of the persistent kernel (kernels.h)
     } lists[2 + kMaxParts - 1];  // [0] squaring blocks (part 0 of a split block), [1] products,
                                  // [2 ..] parts 1 .. of a split block
@@ -100,6 +101,7 @@ struct kc_batch {
     int parts = 3;                // per-pass blocks of 2+ tests in this many parts, one stream each
     int form = -1;                // the form of the captured block graph (BlockForm)
     int graph_parts = 0;          // its number of parts
+    bool graph_narrow = false;    // it launches groups of 4 columns too
     cudaStream_t pstream[kMaxParts] = {};  // [0] is `stream`; [1 ..] the other parts of a split block
     cudaEvent_t fork = nullptr;            // split blocks: the other streams start after it
     cudaEvent_t join[kMaxParts] = {};      //   and `stream` waits for each of theirs
@@ -142,17 +144,24 @@ bool grow_lists(kc_batch *b, kc_batch::Lists &l, int tests, int rows, int cols) 
     free_lists(l);
     l.cap_tests = std::max(tests, 64) * 2;
     l.cap_rows = std::max(rows, 1024) * 2;
-    l.cap_cols = std::max(cols, 1024) * 2;
+    l.cap_cols = std::max(cols, 1024) * 2;  // of each width
     return bok(b, cudaMalloc((void **)&l.d_desc, l.cap_tests * sizeof(TestDesc))) &&
            bok(b, cudaMalloc((void **)&l.d_rows, l.cap_rows * sizeof(WorkItem))) &&
-           bok(b, cudaMalloc((void **)&l.d_cols, l.cap_cols * sizeof(WorkItem))) &&
-           bok(b, cudaMalloc((void **)&l.d_cnt, 2 * sizeof(int))) &&
+           bok(b, cudaMalloc((void **)&l.d_cols, 2 * l.cap_cols * sizeof(WorkItem))) &&
+           bok(b, cudaMalloc((void **)&l.d_cnt, 3 * sizeof(int))) &&
            bok(b, cudaMalloc((void **)&l.d_flow, (kFlowDone + l.cap_tests) * sizeof(unsigned))) &&
            bok(b, cudaMemsetAsync(l.d_flow, 0, (kFlowDone + l.cap_tests) * sizeof(unsigned), b->stream)) &&
            bok(b, cudaMallocHost((void **)&l.h_desc, l.cap_tests * sizeof(TestDesc))) &&
            bok(b, cudaMallocHost((void **)&l.h_rows, l.cap_rows * sizeof(WorkItem))) &&
-           bok(b, cudaMallocHost((void **)&l.h_cols, l.cap_cols * sizeof(WorkItem))) &&
-           bok(b, cudaMallocHost((void **)&l.h_cnt, 2 * sizeof(int)));
+           bok(b, cudaMallocHost((void **)&l.h_cols, 2 * l.cap_cols * sizeof(WorkItem))) &&
+           bok(b, cudaMallocHost((void **)&l.h_cnt, 3 * sizeof(int)));
+}
+
+// any slot with groups of 4 columns (kc_engine_create)
+bool has_narrow(const kc_batch *b) {
+    for (auto &s : b->slots)
+        if (s.used && s.e && s.e->G != kGroup) return true;
+    return false;
 }
 
 LaunchSet launch_set(kc_batch *b, const kc_batch::Lists &l, size_t row_lane, size_t col_smem) {
@@ -165,6 +174,9 @@ LaunchSet launch_set(kc_batch *b, const kc_batch::Lists &l, size_t row_lane, siz
     s.ncols = l.cap_cols;
     s.nrows_dev = l.d_cnt;
     s.ncols_dev = l.d_cnt + 1;
+    s.narrow = has_narrow(b);
+    s.cols4 = l.d_cols + l.cap_cols;
+    s.ncols4_dev = l.d_cnt + 2;
     s.grid_rows = b->grid;
     s.grid_cols = b->grid;
     s.threads = b->threads;
@@ -417,7 +429,7 @@ bool fill_lists(kc_batch *b, kc_batch::Lists &l, const std::vector<Entry> &ents)
         cols += (int)en.s->e->NG;
     }
     if (!grow_lists(b, l, (int)ents.size(), rows, cols)) return false;
-    std::vector<std::pair<int, WorkItem>> rv, cv;
+    std::vector<std::pair<int, WorkItem>> rv, cv, cv4;
     for (size_t t = 0; t < ents.size(); t++) {
         const Entry &en = ents[t];
         TestDesc d = en.s->e->desc;
@@ -433,21 +445,27 @@ bool fill_lists(kc_batch *b, kc_batch::Lists &l, const std::vector<Entry> &ents)
         l.h_desc[t] = d;
         const LengthPlan &P = *en.s->e->plan;
         for (size_t p = 0; p < P.pairs.size(); p++) rv.push_back({(int)P.C, WorkItem{(int)t, (int)p}});
-        for (uint32_t g = 0; g < en.s->e->NG; g++) cv.push_back({(int)P.R, WorkItem{(int)t, (int)g}});
+        auto &cw = en.s->e->G == kGroup ? cv : cv4;
+        for (uint32_t g = 0; g < en.s->e->NG; g++) cw.push_back({(int)P.R, WorkItem{(int)t, (int)g}});
     }
     // longest items first, so the grid-stride walk ends with the short ones
     auto by_size = [](const std::pair<int, WorkItem> &a, const std::pair<int, WorkItem> &c) { return a.first > c.first; };
     std::stable_sort(rv.begin(), rv.end(), by_size);
     std::stable_sort(cv.begin(), cv.end(), by_size);
+    std::stable_sort(cv4.begin(), cv4.end(), by_size);
     for (size_t i = 0; i < rv.size(); i++) l.h_rows[i] = rv[i].second;
     for (size_t i = 0; i < cv.size(); i++) l.h_cols[i] = cv[i].second;
+    for (size_t i = 0; i < cv4.size(); i++) l.h_cols[l.cap_cols + i] = cv4[i].second;
     l.h_cnt[0] = (int)rv.size();
     l.h_cnt[1] = (int)cv.size();
-    b->h2d += ents.size() * sizeof(TestDesc) + (rv.size() + cv.size()) * sizeof(WorkItem) + 2 * sizeof(int);
+    l.h_cnt[2] = (int)cv4.size();
+    b->h2d += ents.size() * sizeof(TestDesc) + (rv.size() + cv.size() + cv4.size()) * sizeof(WorkItem) + 3 * sizeof(int);
     return bok(b, cudaMemcpyAsync(l.d_desc, l.h_desc, ents.size() * sizeof(TestDesc), cudaMemcpyHostToDevice, b->stream)) &&
            bok(b, cudaMemcpyAsync(l.d_rows, l.h_rows, rv.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, b->stream)) &&
            bok(b, cudaMemcpyAsync(l.d_cols, l.h_cols, cv.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, b->stream)) &&
-           bok(b, cudaMemcpyAsync(l.d_cnt, l.h_cnt, 2 * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+           (cv4.empty() || bok(b, cudaMemcpyAsync(l.d_cols + l.cap_cols, l.h_cols + l.cap_cols, cv4.size() * sizeof(WorkItem),
+                                                  cudaMemcpyHostToDevice, b->stream))) &&
+           bok(b, cudaMemcpyAsync(l.d_cnt, l.h_cnt, 3 * sizeof(int), cudaMemcpyHostToDevice, b->stream));
 }
 
 // The forms a block's squarings take: one launch per pass over all slots; the persistent kernel
@@ -472,8 +490,9 @@ kc_batch::Lists &part_lists(kc_batch *b, int p) { return p == 0 ? b->lists[0] : 
 // (re)capture the B-squaring graph when the lists, the shared-memory needs or the form changed
 bool ensure_graph(kc_batch *b, size_t row_lane, size_t col_smem, bool lists_moved, int form, int parts) {
     if (b->graph && !lists_moved && b->graph_B == b->B && row_lane <= b->graph_row_smem &&
-        col_smem <= b->graph_col_smem && form == b->form && parts == b->graph_parts)
+        col_smem <= b->graph_col_smem && form == b->form && parts == b->graph_parts && has_narrow(b) == b->graph_narrow)
         return true;
+    b->graph_narrow = has_narrow(b);
     const kc_batch::Lists &l = b->lists[0];
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -514,7 +533,7 @@ bool ensure_graph(kc_batch *b, size_t row_lane, size_t col_smem, bool lists_move
         for (uint32_t j = 0; j < b->B && launched; j++) {
             for (int p = 0; p < parts; p++) {
                 launch_rows(ps[p], false, nullptr, nullptr, (int)j);
-                launch_col_inverse(ps[p], true, nullptr, (int)j);
+                launch_col_inverse(ps[p], nullptr, (int)j);
                 launch_col_forward(ps[p], nullptr, true, (int)j);
             }
         }
@@ -524,7 +543,7 @@ bool ensure_graph(kc_batch *b, size_t row_lane, size_t col_smem, bool lists_move
     } else {
         for (uint32_t j = 0; j < b->B; j++) {
             launch_rows(s, false, nullptr, nullptr, (int)j);
-            launch_col_inverse(s, true, nullptr, (int)j);
+            launch_col_inverse(s, nullptr, (int)j);
             launch_col_forward(s, nullptr, true, (int)j);
         }
     }
@@ -705,7 +724,7 @@ int kc_batch_step(kc_batch *b, uint32_t blocks, double *gpu_ms) {
         if (sq.empty()) break;
         size_t row_lane, col_smem;
         max_smem(b, row_lane, col_smem);
-        int form = b->persistent ? kPersistent : kPerPass;
+        int form = b->persistent && !has_narrow(b) ? kPersistent : kPerPass;
         const int nparts = form == kPerPass ? std::min<int>(b->parts, (int)sq.size()) : 1;
         if (nparts >= 2) form = kSplit;
         // the lists: all slots in part 0, or a split block's parts of about equal work (row pairs
@@ -752,7 +771,7 @@ int kc_batch_step(kc_batch *b, uint32_t blocks, double *gpu_ms) {
             if (!fill_lists(b, b->lists[1], mu)) return fail(b, "filling the product work lists");
             LaunchSet ms = launch_set(b, b->lists[1], b->graph_row_smem, b->graph_col_smem);
             launch_rows(ms, true, nullptr, nullptr, 0);
-            launch_col_inverse(ms, true, nullptr, 0);
+            launch_col_inverse(ms, nullptr, 0);
             launch_col_forward(ms, nullptr, true, 0);
             bok(b, cudaGetLastError());
         }
@@ -994,7 +1013,7 @@ int kc_batch_profile(kc_batch *b, uint32_t squarings, double *ms, double *flops)
         cudaEventRecord(ev[0], b->stream);
         launch_rows(s, false, nullptr, nullptr, (int)j);
         cudaEventRecord(ev[1], b->stream);
-        launch_col_inverse(s, true, nullptr, (int)j);
+        launch_col_inverse(s, nullptr, (int)j);
         cudaEventRecord(ev[2], b->stream);
         launch_col_forward(s, nullptr, true, (int)j);
         cudaEventRecord(ev[3], b->stream);
@@ -1028,7 +1047,7 @@ int kc_batch_profile_steps(kc_batch *b, uint32_t squarings, double *ms, double *
         const double H = P.H, L = P.L;
         fl += 10.0 * H * std::log2((double)P.C) + 10.0 * L + 2 * (5.0 * H * std::log2((double)P.R) + 7.0 * L);
     }
-    if (sq.empty()) return -1;
+    if (sq.empty() || has_narrow(b)) return -1;
     size_t row_lane, col_smem;
     max_smem(b, row_lane, col_smem);
     row_lane = std::max(row_lane, b->graph_row_smem);

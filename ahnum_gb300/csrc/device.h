@@ -18,22 +18,28 @@
 
 namespace kg {
 
-constexpr int kMaxStages = 12;
+constexpr int kMaxStages = 8;    // of a transform: at most 2048 points, prime factors 2, 3, 5, 7
 constexpr int kGroup = 8;        // widest column group (16 digits per row segment); C is a multiple of it
 constexpr int kMaxAddend = 4;    // sparse constant digits folded into the normaliser
 
-// In-place mixed-radix decimation-in-time transform of length n, unnormalised, input in the
-// digit-reversed order pos() of the plan.  Stage i has radix rad[i] and span
-// span[i] = n / (rad[0]*...*rad[i]); stages run from i = nst-1 (span 1) to 0.  Stage i's
-// twiddle records start at tw + off[i]: for each j < span, rad-1 double2 -- tangent form
-// {tau1, c1} (radix 2), {tau1, tau2}, {tau3, c1}, {c2, c3/c1} (radix 4), or the complex
-// twiddles w^{t*j}, t = 1..rad-1 (odd radices), of w = exp(-2 pi i / (rad*span)).
+// One stage of a transform (fixed_fft.cuh).
+struct alignas(16) FftStage {
+    int radix, span;
+    unsigned magic;    // floor(v / span) = v * magic >> 32 for v < 2^16 (span > 1)
+    int off;           // twiddle records: for each j < span, radix - 1 of w^(t j), t = 1..radix-1,
+                       // w = exp(-2 pi i / (radix span)), each {c1, c0, s1, s0}: the signed 32-bit
+                       // limbs of (c + i s) 2^62
+};
+
+// Mixed-radix transform of length n in 64-bit fixed point, natural order in and out.  The stages run
+// in order, the first with span 1 (no twiddles).
 struct FftPlan {
     int n = 0;
-    int nst = 0;
-    int rad[kMaxStages] = {};
-    int span[kMaxStages] = {};
-    int off[kMaxStages] = {};
+    int ns = 0;        // 2 or more
+    int headroom = 0;  // bits the modulus of the input stays below 2^62
+    int scale = 0;     // the transform leaves a factor 2^-scale
+    int renorm = 0;    // the stage before which the values are scaled up again (0: none)
+    FftStage stage[kMaxStages] = {};
 };
 
 // Everything a kernel needs for one test (one modulus).  Lives in device memory; a kernel copies
@@ -43,24 +49,26 @@ struct alignas(16) TestDesc {
     int L, H, R, C, NG;      // NG = C / G column groups
     int G;                   // columns per column group: 2, 4 or 8 (2G digits per row segment)
     FftPlan rp, cp;          // row plan (length C), column plan (length R)
-    const double2 *twr;      // row stage twiddles
-    const double2 *twc;      // column stage twiddles
-    const double2 *t4;       // [k_r][c] four-step twiddle w_H^{c * k_r}
-    const double2 *sw;       // [k_r][k_c] real-split twiddle w_H^{k_r + R * k_c}
-    const int *posr;         // [r] digit-reversed position of the column transform
-    const int *posc;         // [c] digit-reversed position of the row transform
+    // twiddles, {c1, c0, s1, s0} as in FftPlan
+    const int4 *twr;         // row stages
+    const int4 *twc;         // column stages
+    const int4 *t4;          // [k_r][c] four-step twiddle w_H^{c * k_r}
+    const int4 *sw;          // [k_r][k_c] real-split twiddle w_H^{k_r + R * k_c}
     const int2 *pairs;       // row pairs (k_r, (R - k_r) mod R), k_r <= its partner
     int npairs;
-    // per-modulus tables
+    // per-modulus tables, 64-bit fixed point
     const uint8_t *bits;     // [L]
-    const double *w;         // [L] weights
-    const double *osc;       // [L] k / (w_j * 4H): unweight and scale after a product
-    const double *idig;      // [L] 1 / (R * w_j): unweight after the column inverse alone
+    const long long *w;      // [L] weights w_j 2^61
+    const long long *osc;    // [L] k / (w_j * 4H) 2^(62 - osc_exp): unweight and scale after a product
+    const long long *idig;   // [L] 1 / (R * w_j) 2^(62 - idig_exp): unweight after the column inverse alone
+    int osc_exp, idig_exp;
+    int digit_bits;          // digits entering the column forward pass stay below 2^digit_bits
     // scratch
     long long *dig;          // [L] integer digits between the two column kernels
     long long *slot;         // [NG * R] carry into segment (g, r), index g*R + r
     unsigned long long *maxerr;  // bits of the largest round-off (non-negative double)
-    int *status;             // sticky device-side error flags
+    int *rexp;               // [R] the row pass leaves row k_r as fixed-point numbers times 2^rexp[k_r]
+    int *emax;               // no component of any row of it reaches 2^*emax (INT_MIN between products)
     // top fold
     unsigned long long k;
     int top_t, top_m, top_shift; // top_shift = s_L - s_t

@@ -1,6 +1,8 @@
 // Single-modulus engine behind the kc_* C ABI (include/kite_cuda.h).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -15,10 +17,6 @@
 #include "engine_internal.h"
 
 using namespace kg;
-
-namespace {
-
-}  // namespace
 
 bool kc_ok(kc_engine *e, cudaError_t rc) {
     if (rc != cudaSuccess && !e->err) e->err = -(int)rc;
@@ -82,8 +80,6 @@ bool dalloc(kc_engine *e, T **p, size_t count) {
 }
 
 void release(kc_engine *e) {
-    for (auto &g : e->graphs)
-        if (g.exec) cudaGraphExecDestroy(g.exec);
     cudaFree(e->d_desc);
     cudaFree(e->d_work);
     cudaFree(e->d_bits);
@@ -96,10 +92,32 @@ void release(kc_engine *e) {
     if (e->h_eq) cudaFreeHost(e->h_eq);
     cudaFree(e->d_slot);
     cudaFree(e->d_maxerr);
-    cudaFree(e->d_status);
+    cudaFree(e->d_rexp);
     if (e->h_dig) cudaFreeHost(e->h_dig);
     if (e->h_err) cudaFreeHost(e->h_err);
     if (e->stream) cudaStreamDestroy(e->stream);
+}
+
+// 2^62 m / w for m in [1/2, 1), w in [1, 2) and inv = 1 / w: the quotient of doubles and what its
+// remainder adds
+int64_t fixed_ratio(double m, double w, double inv) {
+    const double q = m * inv, r = std::fma(-q, w, m) * inv;
+    return (int64_t)(q * 0x1p62) + (int64_t)(r * 0x1p62);
+}
+
+// Digits after the deferred carry: balanced, but for the last one of a segment, which takes what is
+// left of a carry of at most 2^52 after the segment's other digits; below 2^(return value).
+int digit_bits(const Layout &lay, int G) {
+    unsigned lo = 64, hi = 0;
+    for (uint8_t b : lay.bits) {
+        lo = b < lo ? b : lo;
+        hi = b > hi ? b : hi;
+    }
+    const int rest = std::max(0, 52 - 2 * G * (int)lo);
+    const int64_t most = ((int64_t)1 << (hi - 1)) + ((int64_t)1 << rest) + 3;
+    int bits = 0;
+    while (((int64_t)1 << bits) <= most) bits++;
+    return bits;
 }
 
 bool upload_desc(kc_engine *e) {
@@ -116,51 +134,44 @@ bool want_err(kc_engine *e) {
 int product(kc_engine *e, double2 *x, const double2 *y) {
     const bool track = want_err(e);
     launch_rows(e->ls, y != nullptr, x, y);
-    launch_col_inverse(e->ls, track, x);
+    launch_col_inverse(e->ls, x, track ? 0 : 1);  // err_every > 1 when this one is not tracked
     launch_col_forward(e->ls, x, true);
     return check_launch(e) ? 0 : e->err;
 }
 
-// A graph of kSquareChunk squarings of x (its kernels take x as an argument); the column
-// inverse tracks round-off on the steps that are multiples of the descriptor's err_every.
-cudaGraphExec_t square_graph(kc_engine *e, double2 *x) {
-    kc_engine::SquareGraph *slot = nullptr;
-    for (auto &g : e->graphs)
-        if (g.exec && g.x == (const double *)x) slot = &g;
-    if (!slot) {
-        slot = &e->graphs[0];
-        for (auto &g : e->graphs)
-            if (!g.exec || g.last_use < slot->last_use) slot = &g;
-        if (slot->exec) cudaGraphExecDestroy(slot->exec);
-        slot->exec = nullptr;
-        slot->x = (const double *)x;
-        cudaGraph_t graph;
-        if (!ok(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal))) return nullptr;
-        for (uint64_t j = 0; j < kSquareChunk; j++) {
-            launch_rows(e->ls, false, x, nullptr, (int)j);
-            launch_col_inverse(e->ls, true, x, (int)j);
-            launch_col_forward(e->ls, x, true, (int)j);
-        }
-        if (!ok(e, cudaStreamEndCapture(e->stream, &graph))) return nullptr;
-        const bool inst = ok(e, cudaGraphInstantiate(&slot->exec, graph, 0));
-        cudaGraphDestroy(graph);
-        if (!inst) return nullptr;
+// Chains wait on their own CTAs, so two of them must not be on the device at once: each one is put
+// behind the previous one of the device, whichever engine launched it.
+struct ChainQueue {
+    std::mutex mu;
+    cudaEvent_t last = nullptr;
+    cudaStream_t stream = nullptr;  // of the last chain
+};
+ChainQueue g_chains[kMaxDevices];
+
+// count squarings of x
+int square_many(kc_engine *e, double2 *x, uint64_t count) {
+    ChainQueue &q = g_chains[e->device];
+    while (count) {
+        const int n = (int)std::min(count, kChainSteps);
+        std::lock_guard<std::mutex> lock(q.mu);
+        if (!q.last && !ok(e, cudaEventCreateWithFlags(&q.last, cudaEventDisableTiming))) return e->err;
+        if (q.stream != e->stream && !ok(e, cudaStreamWaitEvent(e->stream, q.last, 0))) return e->err;
+        if (!ok(e, launch_chain(e->ls, e->chain_grid, x, (int)(e->op_count % e->err_every), n, e->d_chain, e->arrived)) ||
+            !ok(e, cudaEventRecord(q.last, e->stream)))
+            return e->err;
+        q.stream = e->stream;
+        e->arrived += 3u * (unsigned)n * (unsigned)e->chain_grid;
+        e->op_count += (uint64_t)n;
+        count -= (uint64_t)n;
     }
-    slot->last_use = ++e->graph_clock;
-    return slot->exec;
+    return 0;
 }
 
-// count squarings of x: whole chunks from the graph, the rest launched one by one
-int square_many(kc_engine *e, double2 *x, uint64_t count) {
-    while (count >= kSquareChunk) {
-        cudaGraphExec_t g = square_graph(e, x);
-        if (!g || !ok(e, cudaGraphLaunch(g, e->stream))) return e->err ? e->err : -1;
-        count -= kSquareChunk;
-        e->op_count += kSquareChunk;
-    }
-    for (uint64_t i = 0; i < count; i++)
-        if (product(e, x, nullptr)) return e->err;
-    return 0;
+// waits for the engine's queue; false (and sticky) if it failed or a chain's wait gave up
+bool wait_queue(kc_engine *e) {
+    if (!ok(e, cudaStreamSynchronize(e->stream))) return false;
+    if (*(volatile unsigned *)e->h_timeout) ok(e, cudaErrorLaunchTimeout);
+    return !e->err;
 }
 
 int set_addend(kc_engine *e, int64_t c) {
@@ -216,13 +227,14 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         return nullptr;
     }
     const double *wv = w ? w : e->lay.w.data();
-    const double *ov = oscale ? oscale : e->lay.oscale.data();
     // a test run alone spreads each pass over the SMs (shape and column-group width chosen for
     // latency); a batch slot takes the throughput shape and the widest groups
     const unsigned top_digits = e->lay.L - e->lay.top_t;
     if (throughput) {
         e->G = kGroup;
         e->plan = get_plan(L);
+        // a column group's two buffers have to fit shared memory
+        if (e->plan && 2 * (size_t)e->plan->R * e->G * sizeof(longlong2) > kMaxColSmem) e->G = 4;
     } else {
         unsigned min_bits = 64;
         for (uint8_t b : e->lay.bits) min_bits = b < min_bits ? b : min_bits;
@@ -242,32 +254,43 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
     const LengthPlan &P = *e->plan;
     const uint32_t H = P.H;
     e->NG = P.C / e->G;
+    const size_t chain_at = ((size_t)P.R + 2) & ~(size_t)1;  // the chain's words after the exponents, aligned
     bool good = ok(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) &&
                 dalloc(e, &e->d_desc, 1) && dalloc(e, &e->d_work, P.pairs.size() + e->NG) &&
                 dalloc(e, &e->d_bits, L) && dalloc(e, &e->d_w, L) && dalloc(e, &e->d_osc, L) &&
                 dalloc(e, &e->d_idig, L) && dalloc(e, &e->d_dig, L) && dalloc(e, &e->d_dig2, L) &&
                 dalloc(e, &e->d_eq, 1) && ok(e, cudaMallocHost((void **)&e->h_eq, sizeof(int))) &&
                 dalloc(e, &e->d_slot, (size_t)e->NG * P.R) &&
-                dalloc(e, &e->d_maxerr, 1) && dalloc(e, &e->d_status, 1) &&
+                dalloc(e, &e->d_maxerr, 1) && dalloc(e, &e->d_rexp, chain_at + sizeof(ChainCtl) / sizeof(int)) &&
                 ok(e, cudaMallocHost((void **)&e->h_dig, (size_t)L * sizeof(long long))) &&
-                ok(e, cudaMallocHost((void **)&e->h_err, sizeof(unsigned long long)));
+                ok(e, cudaMallocHost((void **)&e->h_err, 2 * sizeof(unsigned long long)));
     if (good) {
-        std::vector<double> osc(L), idig(L);
-        const double s4 = 1.0 / (4.0 * H);
+        std::vector<int64_t> wfix(L), osc(L), idig(L);
+        // k / 4H and 1 / R as m 2^e with m in [1/2, 1)
+        const double ms = std::frexp((double)k / (4.0 * H), &e->desc.osc_exp);
+        const double mi = std::frexp(1.0 / P.R, &e->desc.idig_exp);
         for (uint32_t j = 0; j < L; j++) {
-            osc[j] = ov[j] * s4;
-            idig[j] = 1.0 / ((double)P.R * wv[j]);
+            wfix[j] = (int64_t)(wv[j] * 0x1p61);
+            const double inv = 1.0 / wv[j];
+            osc[j] = fixed_ratio(ms, wv[j], inv);
+            idig[j] = fixed_ratio(mi, wv[j], inv);
         }
+        const int emax0 = INT_MIN;
+        e->h_timeout = reinterpret_cast<unsigned *>(e->h_err + 1);
+        *e->h_timeout = 0;
+        e->d_chain = reinterpret_cast<ChainCtl *>(e->d_rexp + chain_at);
+        const ChainCtl chain0{0, 0, e->h_timeout};
         std::vector<WorkItem> work;
         for (size_t i = 0; i < P.pairs.size(); i++) work.push_back({0, (int)i});
         for (uint32_t g = 0; g < e->NG; g++) work.push_back({0, (int)g});
         good = ok(e, cudaMemcpy(e->d_bits, e->lay.bits.data(), L, cudaMemcpyHostToDevice)) &&
-               ok(e, cudaMemcpy(e->d_w, wv, L * sizeof(double), cudaMemcpyHostToDevice)) &&
-               ok(e, cudaMemcpy(e->d_osc, osc.data(), L * sizeof(double), cudaMemcpyHostToDevice)) &&
-               ok(e, cudaMemcpy(e->d_idig, idig.data(), L * sizeof(double), cudaMemcpyHostToDevice)) &&
+               ok(e, cudaMemcpy(e->d_w, wfix.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
+               ok(e, cudaMemcpy(e->d_osc, osc.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
+               ok(e, cudaMemcpy(e->d_idig, idig.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemcpy(e->d_work, work.data(), work.size() * sizeof(WorkItem), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemset(e->d_maxerr, 0, sizeof(unsigned long long))) &&
-               ok(e, cudaMemset(e->d_status, 0, sizeof(int))) &&
+               ok(e, cudaMemcpy(e->d_rexp + P.R, &emax0, sizeof(int), cudaMemcpyHostToDevice)) &&
+               ok(e, cudaMemcpy(e->d_chain, &chain0, sizeof chain0, cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemset(e->d_slot, 0, (size_t)e->NG * P.R * sizeof(long long)));
     }
     if (good) {
@@ -284,8 +307,6 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         d.twc = P.twc;
         d.t4 = P.t4;
         d.sw = P.sw;
-        d.posr = P.dposr;
-        d.posc = P.dposc;
         d.pairs = P.dpairs;
         d.npairs = (int)P.pairs.size();
         d.bits = e->d_bits;
@@ -295,7 +316,9 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         d.dig = e->d_dig;
         d.slot = e->d_slot;
         d.maxerr = e->d_maxerr;
-        d.status = e->d_status;
+        d.rexp = e->d_rexp;
+        d.emax = e->d_rexp + P.R;
+        d.digit_bits = digit_bits(e->lay, e->G);
         d.k = k;
         d.top_t = (int)e->lay.top_t;
         d.top_m = (int)e->lay.top_m;
@@ -315,10 +338,14 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         s.ncols = (int)e->NG;
         s.grid_rows = s.nrows;
         s.grid_cols = s.ncols;
-        s.row_smem_per_lane = (size_t)P.C * sizeof(double2);
-        s.col_smem = (size_t)P.R * e->G * sizeof(double2);
+        s.row_smem_per_lane = (size_t)P.C * sizeof(longlong2);
+        s.col_smem = 2 * (size_t)P.R * e->G * sizeof(longlong2);
         s.G = e->G;
         good = good && kernels_prepare(s.row_smem_per_lane * 6, s.col_smem) == 0;
+        int nsm = 0;
+        good = good && ok(e, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+        e->chain_grid = good ? chain_grid(s, nsm) : 0;
+        good = e->chain_grid > 0;
     }
     if (!good) {
         release(e);
@@ -361,11 +388,14 @@ void kc_num_free(kc_engine *e, double *x) {
 int kc_from_digits(kc_engine *e, double *x, const int64_t *digits) {
     DeviceGuard dg(e->device);
     const size_t L = e->lay.L;
-    if (!ok(e, cudaStreamSynchronize(e->stream))) return e->err;  // staging buffer reuse
+    if (!wait_queue(e)) return e->err;  // staging buffer reuse
     std::memcpy(e->h_dig, digits, L * sizeof(long long));
+    uint64_t mag = 0;  // bit length of the largest digit
+    for (size_t j = 0; j < L; j++) mag |= (uint64_t)(digits[j] ^ (digits[j] >> 63));
+    const int bits = mag ? 64 - __builtin_clzll(mag) : 1;
     if (!ok(e, cudaMemcpyAsync(e->d_dig, e->h_dig, L * sizeof(long long), cudaMemcpyHostToDevice, e->stream)))
         return e->err;
-    launch_col_forward(e->ls, (double2 *)x, false);
+    launch_col_forward(e->ls, (double2 *)x, false, 0, bits);
     return check_launch(e) ? 0 : e->err;
 }
 
@@ -375,7 +405,7 @@ int kc_to_digits(kc_engine *e, const double *x, int64_t *digits) {
     launch_col_digits(e->ls, (const double2 *)x);
     if (!check_launch(e)) return e->err;
     if (!ok(e, cudaMemcpyAsync(e->h_dig, e->d_dig, L * sizeof(long long), cudaMemcpyDeviceToHost, e->stream)) ||
-        !ok(e, cudaStreamSynchronize(e->stream)))
+        !wait_queue(e))
         return e->err;
     std::memcpy(digits, e->h_dig, L * sizeof(long long));
     return 0;
@@ -386,8 +416,7 @@ int kc_equal(kc_engine *e, const double *a, const double *b) {
     if (a == b) return 1;
     kc_queue_equal(e, e->stream, a, b, e->d_eq);
     if (!check_launch(e) ||
-        !ok(e, cudaMemcpyAsync(e->h_eq, e->d_eq, sizeof(int), cudaMemcpyDeviceToHost, e->stream)) ||
-        !ok(e, cudaStreamSynchronize(e->stream)))
+        !ok(e, cudaMemcpyAsync(e->h_eq, e->d_eq, sizeof(int), cudaMemcpyDeviceToHost, e->stream)) || !wait_queue(e))
         return e->err;
     if (*e->h_eq != 2) return *e->h_eq;
     // the device carry did not settle within its bounds: compare canonical limbs on the host
@@ -438,7 +467,7 @@ double kc_maxerr(kc_engine *e) {
     DeviceGuard dg(e->device);
     if (e->err) return 1.0;
     if (!ok(e, cudaMemcpyAsync(e->h_err, e->d_maxerr, sizeof(unsigned long long), cudaMemcpyDeviceToHost, e->stream)) ||
-        !ok(e, cudaStreamSynchronize(e->stream)))
+        !wait_queue(e))
         return 1.0;
     double v;
     std::memcpy(&v, e->h_err, sizeof v);
@@ -463,7 +492,7 @@ int kc_error(const kc_engine *e) { return e->err; }
 
 int kc_sync(kc_engine *e) {
     DeviceGuard dg(e->device);
-    ok(e, cudaStreamSynchronize(e->stream));
+    wait_queue(e);
     return e->err;
 }
 
@@ -501,6 +530,25 @@ int kc_engine_wait_selftest(kc_engine *e, uint64_t wait_cycles) {
         rc = e->err;
     cudaStreamSynchronize(e->stream);
     cudaFree(flow);
+    if (rc != 1) return rc;
+    // a chain whose CTAs wait for one arrival more than there are, on a scratch number
+    ChainCtl c0{0, 0, e->h_timeout}, c1{};
+    ChainCtl *ctl = nullptr;
+    double *x = kc_num_alloc(e);
+    const int emax0 = INT_MIN;
+    rc = -1;
+    if (x && ok(e, cudaMalloc((void **)&ctl, sizeof(ChainCtl))) &&
+        ok(e, cudaMemcpyAsync(ctl, &c0, sizeof c0, cudaMemcpyHostToDevice, e->stream)) &&
+        ok(e, launch_chain(e->ls, e->chain_grid, (double2 *)x, 0, 1, ctl, 1, (long long)wait_cycles)) &&
+        ok(e, cudaMemcpyAsync(&c1, ctl, sizeof c1, cudaMemcpyDeviceToHost, e->stream)) &&
+        ok(e, cudaMemcpyAsync(e->d_rexp + e->plan->R, &emax0, sizeof emax0, cudaMemcpyHostToDevice, e->stream)) &&
+        ok(e, cudaStreamSynchronize(e->stream)))
+        rc = c1.timeout && *(volatile unsigned *)e->h_timeout ? 1 : 0;
+    else if (e->err)
+        rc = e->err;
+    *e->h_timeout = 0;
+    cudaFree(ctl);
+    if (x) kc_num_free(e, x);
     return rc;
 }
 

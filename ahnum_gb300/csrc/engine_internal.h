@@ -21,12 +21,12 @@ struct kc_engine {
     kg::WorkItem *d_work = nullptr;  // rows then columns
     kg::LaunchSet ls;
     uint8_t *d_bits = nullptr;
-    double *d_w = nullptr, *d_osc = nullptr, *d_idig = nullptr;
+    long long *d_w = nullptr, *d_osc = nullptr, *d_idig = nullptr;  // fixed point (TestDesc)
     long long *d_dig = nullptr, *d_slot = nullptr;
     long long *d_dig2 = nullptr;     // second digit vector of the zero test (kc_equal)
     int *d_eq = nullptr, *h_eq = nullptr;  // its verdict, on the device and pinned
     unsigned long long *d_maxerr = nullptr;
-    int *d_status = nullptr;
+    int *d_rexp = nullptr;           // R row exponents, the test's largest (TestDesc::emax), *d_chain
     long long *h_dig = nullptr;      // pinned staging for digit transfers
     unsigned long long *h_err = nullptr;
     int err = 0;
@@ -36,17 +36,13 @@ struct kc_engine {
     int64_t add_c = 0;
     int G = 8;                       // columns per column group
     uint32_t NG = 0;                 // column groups, C / G
-    // squarings of one number replayed from a CUDA graph (kSquareChunk of them per replay),
-    // one graph per recently squared number
-    struct SquareGraph {
-        const double *x = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        uint64_t last_use = 0;
-    } graphs[4];
-    uint64_t graph_clock = 0;
+    kg::ChainCtl *d_chain = nullptr;   // squaring chains: device words
+    unsigned *h_timeout = nullptr;     //   pinned, after h_err: non-zero once a wait in one gave up
+    unsigned arrived = 0;              //   arrivals at the barrier so far
+    int chain_grid = 0;
 };
 
-constexpr uint64_t kSquareChunk = 16;
+constexpr uint64_t kChainSteps = 512;  // squarings per launch: some 5 ms, 60 ms at the longest lengths
 
 // kc_engine_new for a test run alone (throughput = false: shape and group width chosen for the
 // latency of one squaring) or for a batch slot (throughput = true: the throughput shape, G = 8).

@@ -8,7 +8,8 @@
 namespace kg {
 
 constexpr int kThreads = 256;
-constexpr int kMinBlocks = 4;   // CTAs per SM the pass kernels are compiled for (64 registers)
+constexpr int kMinBlocks = 3;   // CTAs per SM the pass kernels are compiled for (80 registers)
+constexpr size_t kMaxColSmem = 224 * 1024;  // dynamic shared memory a column group may take
 constexpr int kMaxDevices = 64;  // devices tracked by the per-device tables of this library
 
 // Control words of the persistent squaring kernel (device memory, zeroed before each launch):
@@ -31,11 +32,17 @@ struct LaunchSet {
     int ncols = 0;
     const int *nrows_dev = nullptr;    // if set, the item counts are read on the device
     const int *ncols_dev = nullptr;    //   (graphs captured once, lists refilled per launch)
+    // column-group items of tests with groups of 4 in a batch whose other tests have groups of G
+    // (long columns); launched when narrow is set
+    bool narrow = false;
+    const WorkItem *cols4 = nullptr;
+    const int *ncols4_dev = nullptr;
     int grid_rows = 0, grid_cols = 0;
-    size_t row_smem_per_lane = 0;      // C * sizeof(double2) for the longest row
-    size_t col_smem = 0;               // R * G * sizeof(double2) for the longest column
+    size_t row_smem_per_lane = 0;      // C * 16 bytes for the longest row
+    size_t col_smem = 0;               // 2 R G * 16 bytes for the longest column
     int G = kGroup;                    // column-group width of every test in the launch
     int threads = kThreads;            // block size: 256, or 128 for twice the CTAs per SM
+    bool overlap = true;               // programmatic dependent launch (launch.cuh)
 };
 
 // Raise (never lower) the kernels' dynamic shared-memory limits on the current device; 0 on
@@ -45,8 +52,9 @@ int kernels_prepare(size_t row_smem, size_t col_smem);
 // x, y non-null override the per-test operands (single-test use).  `step` is the index of
 // this squaring within a launch sequence: tests whose count is <= step sit it out.
 void launch_rows(const LaunchSet &s, bool mul, double2 *x, const double2 *y, int step = 0);
-void launch_col_inverse(const LaunchSet &s, bool track_err, const double2 *x, int step = 0);
-void launch_col_forward(const LaunchSet &s, double2 *x, bool use_slots, int step = 0);
+void launch_col_inverse(const LaunchSet &s, const double2 *x, int step = 0);
+// digit_bits > 0: the digits stay below 2^digit_bits; 0: they are a product's (TestDesc::digit_bits).
+void launch_col_forward(const LaunchSet &s, double2 *x, bool use_slots, int step = 0, int digit_bits = 0);
 // FP64 FMA throughput probe: `iters` dependent-chain DFMAs per thread over grid x block;
 // the result is written to out[0] only if the chains overflow (never).
 void launch_fp64_probe(cudaStream_t st, int grid, int block, int iters, double *out);
@@ -69,6 +77,26 @@ int launch_squarings(const LaunchSet &s, unsigned *flow, int step0, int nsteps, 
 // stream capture.
 int squarings_grid(const LaunchSet &s, int nsm);
 size_t squarings_smem(size_t row_smem, size_t col_smem);
+// the limit of one file's kernels (kernels_prepare calls them); 0 on success
+int rows_set_smem(size_t bytes);
+int col_inverse_set_smem(size_t bytes);
+int col_forward_set_smem(size_t bytes);
+int squarings_set_smem(size_t bytes);
+// The chain of one test run alone (chain.cu): its CTAs' barrier and the word that says a wait gave up,
+// the latter also in pinned host memory, which the host reads after any synchronisation.
+struct ChainCtl {
+    unsigned arrived;
+    unsigned timeout;
+    unsigned *host_timeout;
+};
+// `nsteps` squarings of x (squaring step0, step0 + 1, ... for the tracking of round-off) in one
+// cooperative launch of `grid` CTAs (chain_grid), which arrive 3 nsteps times each at ctl->arrived,
+// `arrived` before the launch.
+cudaError_t launch_chain(const LaunchSet &s, int grid, double2 *x, int step0, int nsteps, ChainCtl *ctl, unsigned arrived,
+                         long long limit = kWaitCycles);
+// CTAs of a chain: one per item of the larger pass, at most what is resident at once; 0 on failure.
+int chain_grid(const LaunchSet &s, int nsm);
+int chain_set_smem(size_t bytes);
 // op: 0 copy, 1 add, 2 sub
 void launch_elementwise(cudaStream_t st, double2 *x, const double2 *y, size_t n, int op);
 

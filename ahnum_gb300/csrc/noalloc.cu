@@ -104,8 +104,9 @@ extern "C" int kc_square_noalloc(kc_engine *e, const double *x, double *y) {
         if (c == cudaSuccess) {
             LaunchSet s = e->ls;
             s.tests = reinterpret_cast<const TestDesc *>(base);
+            s.overlap = false;  // the descriptor is a kernel's output
             launch_rows(s, false, reinterpret_cast<double2 *>(y), nullptr);
-            launch_col_inverse(s, true, reinterpret_cast<const double2 *>(y));
+            launch_col_inverse(s, reinterpret_cast<const double2 *>(y));
             launch_col_forward(s, reinterpret_cast<double2 *>(y), true);
             c = cudaGetLastError();
         }

@@ -3,10 +3,13 @@
 
 #include <cuda_runtime.h>
 
+#include <climits>
+#include <cstdint>
 #include <cstdlib>
 
 #include "../../include/kite_cuda.h"
 
+#include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -24,8 +27,6 @@ LengthPlan::~LengthPlan() {
     cudaFree(twc);
     cudaFree(t4);
     cudaFree(sw);
-    cudaFree(dposr);
-    cudaFree(dposc);
     cudaFree(dpairs);
     if (prev >= 0) cudaSetDevice(prev);
 }
@@ -171,113 +172,99 @@ bool choose_latency_shape(uint32_t H, int nsm, unsigned min_bits, unsigned top_d
 }
 
 bool make_fft_plan(int n, FftPlan &pl) {
-    // radix 4 throughout the power-of-two part (tangent twiddles), one radix 2 if needed, and
-    // the odd radices last: the last plan stage has span 1 and runs without twiddles, so the
-    // costlier odd butterflies take no twiddle multiplications there.
+    // The odd radices first (the first stage has span 1 and no twiddles), then a radix 2 if needed,
+    // then radix 4; a transform of one stage gets a second one of radix 1.
+    std::vector<int> rad;
+    int m = n;
+    for (int p : {7, 5, 3})
+        for (; m % p == 0; m /= p) rad.push_back(p);
+    int fours = 0;
+    for (; m % 4 == 0; m /= 4) fours++;
+    if (m % 2 == 0) {
+        rad.push_back(2);
+        m /= 2;
+    }
+    if (m != 1 || n < 2) return false;
+    rad.insert(rad.end(), fours, 4);
+    if (rad.size() == 1) rad.push_back(1);
+    if (rad.size() > (size_t)kMaxStages) return false;
     pl = FftPlan{};
     pl.n = n;
-    int m = n, st = 0;
-    auto push = [&](int p) {
-        if (st >= kMaxStages) return false;
-        pl.rad[st++] = p;
-        m /= p;
-        return true;
-    };
-    while (m % 4 == 0)
-        if (!push(4)) return false;
-    if (m % 2 == 0 && !push(2)) return false;
-    for (int p : {3, 5, 7})
-        while (m % p == 0)
-            if (!push(p)) return false;
-    if (m != 1) return false;
-    pl.nst = st;
-    int span = n, off = 0;
-    for (int i = 0; i < st; i++) {
-        span /= pl.rad[i];
-        pl.span[i] = span;
-        pl.off[i] = off;
-        off += (pl.rad[i] - 1) * span;
+    int s = 1, o = 0;
+    double growth = 1, largest = 1;  // of the modulus, stage by stage
+    for (int p : rad) {
+        FftStage &g = pl.stage[pl.ns];
+        g.radix = p;
+        g.span = s;
+        g.magic = s > 1 ? (unsigned)((1ull << 32) / s + 1) : 0;
+        g.off = o;
+        const bool divides = pl.ns > 0 && p > 2;  // a twiddled butterfly of radix 3, 4, 5, 7
+        growth *= divides ? p / 4.0 : p;
+        if (divides) pl.scale += 2;
+        largest = std::max(largest, growth);
+        o += (p - 1) * s;
+        s *= p;
+        pl.ns++;
     }
+    // half a bit for the modulus of two components
+    pl.headroom = (int)std::ceil(std::log2(largest) + 0.5 - 1e-9);
+    // Random data lose half a bit a level against the bound.  Up to four bits of that leave the
+    // round-off below half of what FP64 had at the same length; longer transforms take the bits
+    // back before their last two radix-4 stages, else the loss would pass FP64's from 2^9 points on.
+    if (n > 256 && pl.ns >= 3) pl.renorm = pl.ns - 2;
     return true;
 }
 
-double2 cis_neg(uint64_t j, uint64_t m) {
-    j %= m;
-    // angle pi*x with x = num/den = 2j/m in [0, 2), reduced to [0, 1/4] by exact reflections
-    uint64_t num = 2 * j, den = m;
-    double sc = 1, ss = 1;
-    bool swap = false;
-    if (num > den) {  // cos(pi x) = -cos(pi(x-1)), sin likewise
-        num -= den;
-        sc = -sc;
-        ss = -ss;
-    }
-    if (2 * num > den) {  // x -> 1 - x: cos negates
-        num = den - num;
-        sc = -sc;
-    }
-    if (4 * num > den) {  // x -> 1/2 - x: cos and sin swap
-        num = den - 2 * num;
-        den *= 2;
-        swap = true;
-    }
-    long double th = 3.14159265358979323846264338327950288L * (long double)num / (long double)den;
-    double c = (double)cosl(th), s = (double)sinl(th);
-    if (swap) std::swap(c, s);
-    return make_double2(sc * c, -ss * s);
+// round(v 2^62) in signed limbs; the lower one has a negative
+static void limbs62(long double v, int &hi, int &lo) {
+    int64_t x = (int64_t)std::floor(v * 4611686018427387904.0L + 0.5L);
+    if ((int32_t)(uint32_t)x == INT32_MIN) x++;
+    hi = (int)((x + 0x80000000ll) >> 32);
+    lo = (int)(uint32_t)x;
 }
 
-static void positions(const FftPlan &pl, std::vector<int> &rev, std::vector<int> &pos) {
-    int n = pl.n;
-    rev.assign(n, 0);
-    pos.assign(n, 0);
-    for (int k = 0; k < n; k++) {
-        int kk = k, p = 0;
-        for (int i = 0; i < pl.nst; i++) {
-            p += (kk % pl.rad[i]) * pl.span[i];
-            kk /= pl.rad[i];
+std::vector<int4> roots_neg(uint32_t m) {
+    std::vector<int4> r(m);
+    for (uint32_t j = 0; 2 * j <= m; j++) {
+        // angle pi*x with x = num/den = 2j/m in [0, 1], reduced to [0, 1/4] by exact reflections
+        uint64_t num = 2 * (uint64_t)j, den = m;
+        bool neg = false, swap = false;
+        if (2 * num > den) {  // x -> 1 - x: cos negates
+            num = den - num;
+            neg = true;
         }
-        pos[k] = p;
-        rev[p] = k;
+        if (4 * num > den) {  // x -> 1/2 - x: cos and sin swap
+            num = den - 2 * num;
+            den *= 2;
+            swap = true;
+        }
+        const long double th = 3.14159265358979323846264338327950288L * (long double)num / (long double)den;
+        long double c = cosl(th), s = sinl(th);
+        if (swap) std::swap(c, s);
+        if (neg) c = -c;
+        limbs62(c, r[j].x, r[j].y);
+        limbs62(-s, r[j].z, r[j].w);
+        if (j) {
+            r[m - j] = r[j];
+            limbs62(s, r[m - j].z, r[m - j].w);
+        }
     }
+    return r;
 }
 
-// Twiddle records of every stage (see FftPlan): tangent form for radix 2 and 4, complex
-// twiddles for the odd radices.  A cosine that is exactly 0 is replaced by 2^-60 (and the
-// tangent scaled to match), which changes the product by far less than one ulp.
-static void stage_twiddles(const FftPlan &pl, std::vector<double2> &tw) {
+// Twiddle records of every stage (see FftStage), from the roots of order h, a multiple of pl.n
+static void stage_twiddles(const FftPlan &pl, const std::vector<int4> &roots, std::vector<int4> &tw) {
+    const uint64_t h = roots.size();
     tw.clear();
-    const double tiny = std::ldexp(1.0, -60);
-    for (int i = 0; i < pl.nst; i++) {
-        const int p = pl.rad[i], s = pl.span[i], sz = p * s;
-        for (int j = 0; j < s; j++) {
-            double c[4] = {1, 1, 1, 1}, tau[4] = {0, 0, 0, 0};
-            double2 w[8];
-            for (int t = 1; t < p; t++) {
-                w[t] = cis_neg((uint64_t)t * j, (uint64_t)sz);
-                double cc = w[t].x;
-                if (cc == 0.0) cc = tiny;
-                if (t < 4) {
-                    c[t] = cc;
-                    tau[t] = w[t].y / cc;
-                }
-            }
-            if (p == 2) {
-                tw.push_back(make_double2(tau[1], c[1]));
-            } else if (p == 4) {
-                tw.push_back(make_double2(tau[1], tau[2]));
-                tw.push_back(make_double2(tau[3], c[1]));
-                tw.push_back(make_double2(c[2], c[3] / c[1]));
-            } else {
-                for (int t = 1; t < p; t++) tw.push_back(w[t]);
-            }
-        }
+    for (int i = 0; i < pl.ns; i++) {
+        const int p = pl.stage[i].radix, s = pl.stage[i].span;
+        const uint64_t step = h / ((uint64_t)p * s);
+        for (int j = 0; j < s; j++)
+            for (int t = 1; t < p; t++) tw.push_back(roots[step * t * j]);
     }
 }
 
-std::shared_ptr<LengthPlan> build_plan_host(uint32_t L, uint32_t rows, std::vector<double2> *twr,
-                                            std::vector<double2> *twc, std::vector<double2> *t4,
-                                            std::vector<double2> *sw) {
+std::shared_ptr<LengthPlan> build_plan_host(uint32_t L, uint32_t rows, PlanTables *tables) {
     if (L % (2 * kGroup) || L < 64) return nullptr;
     auto pl = std::make_shared<LengthPlan>();
     pl->L = L;
@@ -290,25 +277,22 @@ std::shared_ptr<LengthPlan> build_plan_host(uint32_t L, uint32_t rows, std::vect
         return nullptr;
     }
     if (!make_fft_plan((int)pl->C, pl->rp) || !make_fft_plan((int)pl->R, pl->cp)) return nullptr;
-    positions(pl->rp, pl->rev_c, pl->pos_c);
-    positions(pl->cp, pl->rev_r, pl->pos_r);
     const uint32_t R = pl->R, C = pl->C, H = pl->H;
     for (uint32_t kr = 0; kr < R; kr++) {
         uint32_t k2 = (R - kr) % R;
         if (kr <= k2) pl->pairs.push_back(make_int2((int)kr, (int)k2));
     }
-    if (twr) stage_twiddles(pl->rp, *twr);
-    if (twc) stage_twiddles(pl->cp, *twc);
-    if (t4) {
-        t4->resize((size_t)R * C);
+    if (tables) {
+        const std::vector<int4> roots = roots_neg(H);
+        stage_twiddles(pl->rp, roots, tables->twr);
+        stage_twiddles(pl->cp, roots, tables->twc);
+        tables->t4.resize((size_t)R * C);
+        tables->sw.resize((size_t)R * C);
         for (uint32_t kr = 0; kr < R; kr++)
-            for (uint32_t c = 0; c < C; c++) (*t4)[(size_t)kr * C + c] = cis_neg((uint64_t)c * kr % H, H);
-    }
-    if (sw) {
-        sw->resize((size_t)R * C);
-        for (uint32_t kr = 0; kr < R; kr++)
-            for (uint32_t kc = 0; kc < C; kc++)
-                (*sw)[(size_t)kr * C + kc] = cis_neg(((uint64_t)kr + (uint64_t)R * kc) % H, H);
+            for (uint32_t c = 0; c < C; c++) {
+                tables->t4[(size_t)kr * C + c] = roots[(uint64_t)c * kr % H];
+                tables->sw[(size_t)kr * C + c] = roots[kr + (uint64_t)R * c];
+            }
     }
     return pl;
 }
@@ -331,13 +315,12 @@ std::shared_ptr<LengthPlan> get_plan(uint32_t L, uint32_t R) {
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find({dev, L, R});
     if (it != cache.end()) return it->second;
-    std::vector<double2> twr, twc, t4, sw;
-    auto pl = build_plan_host(L, R, &twr, &twc, &t4, &sw);
+    PlanTables t;
+    auto pl = build_plan_host(L, R, &t);
     if (!pl) return nullptr;
     pl->device = dev;
-    bool ok = upload(twr, &pl->twr, pl->device_bytes) && upload(twc, &pl->twc, pl->device_bytes) &&
-              upload(t4, &pl->t4, pl->device_bytes) && upload(sw, &pl->sw, pl->device_bytes) &&
-              upload(pl->pos_r, &pl->dposr, pl->device_bytes) && upload(pl->pos_c, &pl->dposc, pl->device_bytes) &&
+    bool ok = upload(t.twr, &pl->twr, pl->device_bytes) && upload(t.twc, &pl->twc, pl->device_bytes) &&
+              upload(t.t4, &pl->t4, pl->device_bytes) && upload(t.sw, &pl->sw, pl->device_bytes) &&
               upload(pl->pairs, &pl->dpairs, pl->device_bytes);
     if (!ok) return nullptr;
     cache[{dev, L, R}] = pl;

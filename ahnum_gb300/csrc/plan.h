@@ -13,13 +13,10 @@ namespace kg {
 struct LengthPlan {
     uint32_t L = 0, H = 0, R = 0, C = 0;
     FftPlan rp, cp;                   // row plan (C points), column plan (R points)
-    std::vector<int> rev_r, pos_r;    // DIF output position <-> frequency, column transform
-    std::vector<int> rev_c, pos_c;    // same for the row transform
     std::vector<int2> pairs;          // row pairs (p, p'), p <= p'
     // device copies
     int device = -1;
-    double2 *twr = nullptr, *twc = nullptr, *t4 = nullptr, *sw = nullptr;
-    int *dposr = nullptr, *dposc = nullptr;
+    int4 *twr = nullptr, *twc = nullptr, *t4 = nullptr, *sw = nullptr;
     int2 *dpairs = nullptr;
     size_t device_bytes = 0;
     ~LengthPlan();
@@ -32,11 +29,11 @@ bool choose_shape(uint32_t H, uint32_t &R, uint32_t &C);
 bool set_shape_override(uint32_t L, uint32_t R);
 // Usable shapes of H = R*C near balance, at most `max`; returns the count.
 int shape_candidates(uint32_t H, uint32_t *R, uint32_t *C, int max);
-// Radices for a length-n transform in DIF order; false if n has a prime factor above 7.
+// The stages of a length-n transform; false if n has a prime factor above 7.
 bool make_fft_plan(int n, FftPlan &pl);
 
-// exp(-2 pi i j / m) with the angle reduced exactly in integer arithmetic
-double2 cis_neg(uint64_t j, uint64_t m);
+// exp(-2 pi i j / m), j = 0..m-1, times 2^62 in limbs {c1, c0, s1, s0} (FftStage)
+std::vector<int4> roots_neg(uint32_t m);
 
 // Shape and column-group width for one test run alone: spread every pass over the SMs so the
 // squaring's latency, not its total FP64 work, is smallest.  Throughput (batched) use takes
@@ -53,8 +50,9 @@ bool set_latency_override(uint32_t L, uint32_t R, int G);
 // the device upload fails.  Thread-safe.
 std::shared_ptr<LengthPlan> get_plan(uint32_t L, uint32_t R = 0);
 // Host tables only (no device upload).
-std::shared_ptr<LengthPlan> build_plan_host(uint32_t L, uint32_t R, std::vector<double2> *twr,
-                                            std::vector<double2> *twc, std::vector<double2> *t4,
-                                            std::vector<double2> *sw);
+struct PlanTables {
+    std::vector<int4> twr, twc, t4, sw;
+};
+std::shared_ptr<LengthPlan> build_plan_host(uint32_t L, uint32_t R, PlanTables *tables);
 
 }  // namespace kg
