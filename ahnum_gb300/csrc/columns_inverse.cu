@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_col_inverse(const Test
     walk_items(
         tests, work, nwork, step, &s_desc, &s_ctl,
         [](const TestDesc &T, int g) { touch_columns(T, g, T.osc); },
-        [&](const TestDesc &T, int g) { col_inverse_item<LG>(T, g, step, xo ? xo : T.x, sm, s_ctl); });
+        [&](const TestDesc &T, int g) { col_inverse_item<LG, GlobalTables>(T, g, step, xo ? xo : T.x, sm, s_ctl); });
 }
 
 template <int LG>
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_col_digits(const TestD
     walk_items(
         tests, work, nwork, 0, &s_desc, &s_ctl,
         [](const TestDesc &T, int g) { touch_columns(T, g, T.idig); },
-        [&](const TestDesc &T, int g) { col_digits_item<LG>(T, g, xo ? xo : T.x, digo ? digo : T.dig, sm, s_ctl); });
+        [&](const TestDesc &T, int g) { col_digits_item<LG, GlobalTables>(T, g, xo ? xo : T.x, digo ? digo : T.dig, sm, s_ctl); });
 }
 
 void launch_col_inverse(const LaunchSet &s, const double2 *x, int step) {

@@ -62,6 +62,7 @@ struct alignas(16) TestDesc {
     const long long *osc;    // [L] k / (w_j * 4H) 2^(62 - osc_exp): unweight and scale after a product
     const long long *idig;   // [L] 1 / (R * w_j) 2^(62 - idig_exp): unweight after the column inverse alone
     int osc_exp, idig_exp;
+    int pitch;               // columns from one row to the next of t4, osc, w and bits: C
     int digit_bits;          // digits entering the column forward pass stay below 2^digit_bits
     // scratch
     long long *dig;          // [L] integer digits between the two column kernels
@@ -70,7 +71,7 @@ struct alignas(16) TestDesc {
     int *rexp;               // [R] the row pass leaves row k_r as fixed-point numbers times 2^rexp[k_r]
     int *emax;               // no component of any row of it reaches 2^*emax (INT_MIN between products)
     // top fold
-    unsigned long long k;
+    unsigned long long k, k_inv; // k_inv = floor((2^64 - 1) / k)
     int top_t, top_m, top_shift; // top_shift = s_L - s_t
     // constant digits added before the carry (LLR: -2), (index, value)
     int nadd;

@@ -156,7 +156,7 @@ int square_many(kc_engine *e, double2 *x, uint64_t count) {
         std::lock_guard<std::mutex> lock(q.mu);
         if (!q.last && !ok(e, cudaEventCreateWithFlags(&q.last, cudaEventDisableTiming))) return e->err;
         if (q.stream != e->stream && !ok(e, cudaStreamWaitEvent(e->stream, q.last, 0))) return e->err;
-        if (!ok(e, launch_chain(e->ls, e->chain_grid, x, (int)(e->op_count % e->err_every), n, e->d_chain, e->arrived)) ||
+        if (!ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, x, (int)(e->op_count % e->err_every), n, e->d_chain, e->arrived)) ||
             !ok(e, cudaEventRecord(q.last, e->stream)))
             return e->err;
         q.stream = e->stream;
@@ -318,8 +318,10 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         d.maxerr = e->d_maxerr;
         d.rexp = e->d_rexp;
         d.emax = e->d_rexp + P.R;
+        d.pitch = (int)P.C;
         d.digit_bits = digit_bits(e->lay, e->G);
         d.k = k;
+        d.k_inv = ~0ull / k;
         d.top_t = (int)e->lay.top_t;
         d.top_m = (int)e->lay.top_m;
         d.top_shift = (int)(e->lay.sL - e->lay.top_st);
@@ -341,10 +343,11 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         s.row_smem_per_lane = (size_t)P.C * sizeof(longlong2);
         s.col_smem = 2 * (size_t)P.R * e->G * sizeof(longlong2);
         s.G = e->G;
-        good = good && kernels_prepare(s.row_smem_per_lane * 6, s.col_smem) == 0;
-        int nsm = 0;
-        good = good && ok(e, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-        e->chain_grid = good ? chain_grid(s, nsm) : 0;
+        // twiddles of both plans, split twiddles of a row; t4, osc, w of a column group, its widths
+        s.table_smem = ((size_t)2 * P.C + P.R + 3 * (size_t)P.R * e->G) * 16 + ((size_t)2 * P.R * e->G + 15) / 16 * 16;
+        good = good && ok(e, cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device)) &&
+               kernels_prepare(s.row_smem_per_lane * 6, s.col_smem, chain_smem(s, e->nsm)) == 0;
+        e->chain_grid = good ? chain_grid(s, e->nsm) : 0;
         good = e->chain_grid > 0;
     }
     if (!good) {
@@ -539,7 +542,7 @@ int kc_engine_wait_selftest(kc_engine *e, uint64_t wait_cycles) {
     rc = -1;
     if (x && ok(e, cudaMalloc((void **)&ctl, sizeof(ChainCtl))) &&
         ok(e, cudaMemcpyAsync(ctl, &c0, sizeof c0, cudaMemcpyHostToDevice, e->stream)) &&
-        ok(e, launch_chain(e->ls, e->chain_grid, (double2 *)x, 0, 1, ctl, 1, (long long)wait_cycles)) &&
+        ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, (double2 *)x, 0, 1, ctl, 1, (long long)wait_cycles)) &&
         ok(e, cudaMemcpyAsync(&c1, ctl, sizeof c1, cudaMemcpyDeviceToHost, e->stream)) &&
         ok(e, cudaMemcpyAsync(e->d_rexp + e->plan->R, &emax0, sizeof emax0, cudaMemcpyHostToDevice, e->stream)) &&
         ok(e, cudaStreamSynchronize(e->stream)))

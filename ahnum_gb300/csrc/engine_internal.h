@@ -39,7 +39,7 @@ struct kc_engine {
     kg::ChainCtl *d_chain = nullptr;   // squaring chains: device words
     unsigned *h_timeout = nullptr;     //   pinned, after h_err: non-zero once a wait in one gave up
     unsigned arrived = 0;              //   arrivals at the barrier so far
-    int chain_grid = 0;
+    int chain_grid = 0, nsm = 0;
 };
 
 constexpr uint64_t kChainSteps = 512;  // squarings per launch: some 5 ms, 60 ms at the longest lengths

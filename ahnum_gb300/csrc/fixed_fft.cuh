@@ -36,15 +36,16 @@ namespace kg {
 // the upper limb of v = hi32(v) 2^32 + lo32(v) with both limbs signed
 __device__ __forceinline__ int lo32(long long v) { return (int)v; }
 __device__ __forceinline__ int hi32(long long v) { return (int)(v >> 32) + (int)((unsigned)v >> 31); }
-// a b + c, one multiply-add.  Spelled out: from the C expression the compiler made several
-// instructions, 100 clocks a complex product instead of 59.
-__device__ __forceinline__ long long madw(int a, int b, long long c) {
+// The 64-bit product of two limbs.  Spelled out, so that it is not joined with the add that follows
+// to one multiply-add: that one takes 5.2 clocks a warp and sub-partition (10.4 with a single warp to
+// issue), the product and the add 4.25 (6.1).
+__device__ __forceinline__ long long mulw(int a, int b) {
 #ifdef __CUDA_ARCH__
     long long d;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    asm("mul.wide.s32 %0, %1, %2;" : "=l"(d) : "r"(a), "r"(b));
     return d;
 #else
-    return (long long)a * b + c;
+    return (long long)a * b;
 #endif
 }
 
@@ -86,9 +87,9 @@ struct Acc {
     long long p = 0, t;
     __device__ __forceinline__ explicit Acc(long long half = kHalf) : t(half) {}
     __device__ __forceinline__ void mac(int a1, int a0, int b1, int b0) {
-        t = madw(a1, b0, t);
-        t = madw(a0, b1, t);
-        p = madw(a1, b1, p);
+        t += mulw(a1, b0);
+        t += mulw(a0, b1);
+        p += mulw(a1, b1);
     }
     __device__ __forceinline__ long long high() const { return p + (t >> 32); }
     // four times as much, rounded at the last place of that
@@ -208,20 +209,35 @@ __device__ __forceinline__ longlong2 quarter(longlong2 a, long long half) {
     return make_longlong2((a.x + k) >> 2, (a.y + k) >> 2);
 }
 
+// How a pass reads the tables: in global memory (the read-only path), or wherever they are (the chain
+// keeps its own slices in shared memory).
+struct GlobalTables {
+    template <class V>
+    static __device__ __forceinline__ V load(const V *p) {
+        return __ldg(p);
+    }
+};
+struct AnyTables {
+    template <class V>
+    static __device__ __forceinline__ V load(const V *p) {
+        return *p;
+    }
+};
+
 // One radix-P butterfly of a stage with twiddle records w^t, t = 1..P-1 (tw).  UNIT: the stage of
 // span 1, whose twiddles are 1.  A twiddled butterfly of radix 3, 4, 5 or 7 divides by 4, the others
 // do not scale.
-template <int P, bool INV, bool UNIT>
-__device__ __forceinline__ void butterfly(longlong2 *x, const int4 *__restrict__ tw, long long half) {
+template <int P, bool INV, bool UNIT, class TAB>
+__device__ __forceinline__ void butterfly(longlong2 *x, const int4 *tw, long long half) {
     if constexpr (!UNIT) {
         if constexpr (P == 2) {
-            const int4 w = __ldg(tw);  // unscaled
+            const int4 w = TAB::load(tw);  // unscaled
             x[1] = cmul4(x[1], INV ? conj_tw(w) : w);
         } else {
             x[0] = quarter(x[0], half);
 #pragma unroll
             for (int t = 1; t < P; t++) {
-                const int4 w = __ldg(tw + t - 1);
+                const int4 w = TAB::load(tw + t - 1);
                 x[t] = cmul(x[t], INV ? conj_tw(w) : w, half);
             }
         }
@@ -232,8 +248,8 @@ __device__ __forceinline__ void butterfly(longlong2 *x, const int4 *__restrict__
 // One stage over 2^LG interleaved sequences, element e of sequence l at (e << LG) + l of the buffers.
 // ld(at, e, l) gives the element (at: its index in the source), st(at, e, l, v) takes the result (at:
 // its index in the destination).  Bit l of `odd` draws the rounding of sequence l (half_of).
-template <int P, int LG, bool INV, bool FIRST, class LD, class ST>
-__device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const int4 *__restrict__ tw, unsigned odd,
+template <int P, int LG, bool INV, bool FIRST, class TAB, class LD, class ST>
+__device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const int4 *tw, unsigned odd,
                                           LD &&ld, ST &&st) {
     const int np = n / P, total = np << LG;
     for (int i = threadIdx.x; i < total; i += blockDim.x) {
@@ -243,7 +259,7 @@ __device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const
         longlong2 x[P];
 #pragma unroll
         for (int t = 0; t < P; t++) x[t] = ld(i + t * total, e + t * np, l);
-        if constexpr (P > 1) butterfly<P, INV, FIRST>(x, tw + k * (P - 1), half_of((odd >> l) & 1));
+        if constexpr (P > 1) butterfly<P, INV, FIRST, TAB>(x, tw + k * (P - 1), half_of((odd >> l) & 1));
         const int o = e + blk * (P - 1) * span;
 #pragma unroll
         for (int t = 0; t < P; t++) st((((o + t * span) << LG) + l), o + t * span, l, x[t]);
@@ -251,17 +267,17 @@ __device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const
 }
 
 // The stage of radix p; the last stage of a short transform may have radix 1.
-template <int LG, bool INV, bool FIRST, bool LAST, class LD, class ST>
+template <int LG, bool INV, bool FIRST, bool LAST, class TAB, class LD, class ST>
 __device__ __forceinline__ void dispatch_stage(int n, const FftStage &g, const int4 *tw, unsigned odd, LD &&ld, ST &&st) {
     const int p = g.radix, span = g.span;
     const unsigned magic = g.magic;
     tw += g.off;
 #define KG_STAGE(P)                                                          \
     case P:                                                                  \
-        run_stage<P, LG, INV, FIRST>(n, span, magic, tw, odd, ld, st);       \
+        run_stage<P, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, st);       \
         break;
     if (p == 4) {
-        run_stage<4, LG, INV, FIRST>(n, span, magic, tw, odd, ld, st);
+        run_stage<4, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, st);
         return;
     }
     switch (p) {
@@ -270,7 +286,7 @@ __device__ __forceinline__ void dispatch_stage(int n, const FftStage &g, const i
         KG_STAGE(5)
         KG_STAGE(7)
     default:
-        if constexpr (LAST) run_stage<1, LG, INV, FIRST>(n, span, magic, tw, odd, ld, st);
+        if constexpr (LAST) run_stage<1, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, st);
         break;
     }
 #undef KG_STAGE

@@ -9,6 +9,38 @@
 
 namespace kg {
 
+// Fold of the top region held in dig[top_t..L-1] plus the carry cy at 2^{s_L}
+// (reference src/ctx.c:345-375); returns the amount for digit 0.
+__device__ __forceinline__ long long fold_top(const TestDesc &T, long long *dig, long long cy) {
+    const int L = T.L, t = T.top_t;
+    __int128 H = (__int128)cy << T.top_shift;
+    int pos = 0;
+    for (int j = t; j < L; j++) {
+        H += (__int128)dig[j] << pos;
+        pos += T.bits[j];
+    }
+    const int m = T.top_m;
+    const __int128 K = (__int128)T.k;
+    __int128 lo = H & (((__int128)1 << m) - 1);
+    __int128 hi = H >> m;
+    __int128 rem;
+    __int128 q = floor_div_inv(hi, T.k, T.k_inv, rem);
+    __int128 top = lo + (rem << m);
+    const __int128 span = K << m;
+    if (2 * top >= span) {
+        top -= span;
+        q += 1;
+    }
+    for (int j = t; j + 1 < L; j++) {
+        const int b = T.bits[j];
+        __int128 qq = (top + ((__int128)1 << (b - 1))) >> b;
+        dig[j] = (long long)(top - (qq << b));
+        top = qq;
+    }
+    if (t < L) dig[L - 1] = (long long)top;
+    return (long long)q;
+}
+
 // Zero test of a - b modulo N for two digit vectors of one test (the digits of two numbers, as
 // k_col_digits leaves them): the Gerbicz check's comparison d == x0 * t^(2^B) and the tail's
 // x == t, done where the numbers live.  The reference compares canonical limbs on the host
@@ -135,9 +167,10 @@ __global__ void k_elementwise(double2 *x, const double2 *y, size_t n, int op) {
 // The limit is a property of each kernel in the device's context, shared by every engine and
 // batch of the process, so it only ever grows: lowering it for a small length would make later
 // launches (or captured graphs) of a longer length fail.
-int kernels_prepare(size_t row_smem, size_t col_smem) {
+int kernels_prepare(size_t row_smem, size_t col_smem, size_t chain_smem) {
     static std::mutex mu;
     static size_t row_hw[kMaxDevices] = {}, col_hw[kMaxDevices] = {}, sq_hw[kMaxDevices] = {};
+    static size_t chain_hw[kMaxDevices] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
     std::lock_guard<std::mutex> lock(mu);
@@ -153,8 +186,13 @@ int kernels_prepare(size_t row_smem, size_t col_smem) {
     }
     const size_t sq_smem = squarings_smem(row_smem, col_smem);
     if (sq_smem > sq_hw[dev]) {
-        const int r2 = squarings_set_smem(sq_smem) | chain_set_smem(sq_smem);
+        const int r2 = squarings_set_smem(sq_smem);
         if (!r2) sq_hw[dev] = sq_smem;
+        rc |= r2;
+    }
+    if (chain_smem > chain_hw[dev]) {
+        const int r2 = chain_set_smem(chain_smem);
+        if (!r2) chain_hw[dev] = chain_smem;
         rc |= r2;
     }
     return rc;

@@ -9,6 +9,7 @@ namespace kg {
 
 constexpr int kThreads = 256;
 constexpr int kMinBlocks = 3;   // CTAs per SM the pass kernels are compiled for (80 registers)
+constexpr size_t kMaxChainSmem = 220 * 1024;  // dynamic shared memory of a chain that keeps its tables
 constexpr size_t kMaxColSmem = 224 * 1024;  // dynamic shared memory a column group may take
 constexpr int kMaxDevices = 64;  // devices tracked by the per-device tables of this library
 
@@ -40,6 +41,7 @@ struct LaunchSet {
     int grid_rows = 0, grid_cols = 0;
     size_t row_smem_per_lane = 0;      // C * 16 bytes for the longest row
     size_t col_smem = 0;               // 2 R G * 16 bytes for the longest column
+    size_t table_smem = 0;             // one test: a row pair's and a column group's tables (chain.cu)
     int G = kGroup;                    // column-group width of every test in the launch
     int threads = kThreads;            // block size: 256, or 128 for twice the CTAs per SM
     bool overlap = true;               // programmatic dependent launch (launch.cuh)
@@ -47,7 +49,7 @@ struct LaunchSet {
 
 // Raise (never lower) the kernels' dynamic shared-memory limits on the current device; 0 on
 // success.
-int kernels_prepare(size_t row_smem, size_t col_smem);
+int kernels_prepare(size_t row_smem, size_t col_smem, size_t chain_smem = 0);
 
 // x, y non-null override the per-test operands (single-test use).  `step` is the index of
 // this squaring within a launch sequence: tests whose count is <= step sit it out.
@@ -92,10 +94,11 @@ struct ChainCtl {
 // `nsteps` squarings of x (squaring step0, step0 + 1, ... for the tracking of round-off) in one
 // cooperative launch of `grid` CTAs (chain_grid), which arrive 3 nsteps times each at ctl->arrived,
 // `arrived` before the launch.
-cudaError_t launch_chain(const LaunchSet &s, int grid, double2 *x, int step0, int nsteps, ChainCtl *ctl, unsigned arrived,
+cudaError_t launch_chain(const LaunchSet &s, int nsm, int grid, double2 *x, int step0, int nsteps, ChainCtl *ctl, unsigned arrived,
                          long long limit = kWaitCycles);
 // CTAs of a chain: one per item of the larger pass, at most what is resident at once; 0 on failure.
 int chain_grid(const LaunchSet &s, int nsm);
+size_t chain_smem(const LaunchSet &s, int nsm);  // its dynamic shared memory
 int chain_set_smem(size_t bytes);
 // op: 0 copy, 1 add, 2 sub
 void launch_elementwise(cudaStream_t st, double2 *x, const double2 *y, size_t n, int op);

@@ -116,12 +116,12 @@ __device__ __forceinline__ int clamp_scale(int s) { return max(-900, min(900, s)
 // calls last_st(dst, at, e, l, v), dst being the buffer it may write to (the value returned).
 // Long transforms are scaled to their largest component once more on the way (FftPlan::renorm,
 // *mid a zeroed word of the block) by 2^shift, set before the last stage.  Ends with a barrier.
-template <int LG, bool INV, class LD, class ST>
+template <int LG, bool INV, class TAB, class LD, class ST>
 __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *tw, longlong2 *to, longlong2 *alt,
                                                 unsigned odd, LD &&first_ld, ST &&last_st, unsigned *mid, int &shift) {
     const int n = pl.n, last = pl.ns - 1, renorm = pl.renorm;
     shift = 0;
-    dispatch_stage<LG, INV, true, false>(n, pl.stage[0], tw, odd, first_ld,
+    dispatch_stage<LG, INV, true, false, TAB>(n, pl.stage[0], tw, odd, first_ld,
                                          [&](int at, int, int, longlong2 v) { to[at] = v; });
     __syncthreads();
     for (int i = 1; i < last; i++) {
@@ -133,7 +133,7 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
             const int sh = i == renorm ? shift : 0;
             const bool track = i + 1 == renorm;
             unsigned mag = 0;
-            dispatch_stage<LG, INV, false, false>(
+            dispatch_stage<LG, INV, false, false, TAB>(
                 n, pl.stage[i], tw, odd, [&](int at, int, int) { return cshl(from[at], sh); },
                 [&](int at, int, int, longlong2 v) {
                     to[at] = v;
@@ -143,12 +143,12 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
             __syncthreads();
             if (track) shift = 29 - bit_length(*mid);  // components below 2^61
         } else {
-            dispatch_stage<LG, INV, false, false>(n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; },
+            dispatch_stage<LG, INV, false, false, TAB>(n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; },
                                                   [&](int at, int, int, longlong2 v) { to[at] = v; });
             __syncthreads();
         }
     }
-    dispatch_stage<LG, INV, false, true>(n, pl.stage[last], tw, ~odd, [&](int at, int, int) { return to[at]; },
+    dispatch_stage<LG, INV, false, true, TAB>(n, pl.stage[last], tw, ~odd, [&](int at, int, int) { return to[at]; },
                                          [&](int at, int e, int l, longlong2 v) { last_st(alt, at, e, l, v); });
     __syncthreads();
     return alt;
@@ -216,6 +216,7 @@ __device__ __forceinline__ void split_pair(longlong2 &a, longlong2 &b, int4 w, l
 // A row pair of a number into `raw` as it is in memory, lane 0 row k_r and lane 1 row R-k_r, and its
 // forward transform, from `raw` to `other` and back.  Returns the buffer with the result; `scale` is
 // the power of two it was scaled by, *mag the OR of its components' upper words.  Barriers included.
+template <class TAB>
 __device__ __forceinline__ longlong2 *rows_forward(const TestDesc &T, int2 pr, const double2 *xd, longlong2 *raw,
                                                    longlong2 *other, unsigned odd, unsigned *top, unsigned *mag,
                                                    unsigned *mid, int &scale) {
@@ -236,7 +237,7 @@ __device__ __forceinline__ longlong2 *rows_forward(const TestDesc &T, int2 pr, c
     const int s = clamp_scale(62 - pl.headroom - top_exponent(*top));
     unsigned m = 0;
     int shift;
-    longlong2 *out = transform<1, false>(
+    longlong2 *out = transform<1, false, TAB>(
         pl, T.twr, other, raw, odd,
         [&](int at, int, int) {
             const longlong2 d = raw[at];
@@ -254,7 +255,7 @@ __device__ __forceinline__ longlong2 *rows_forward(const TestDesc &T, int2 pr, c
 }
 
 // One row pair of one test.  Ends with a barrier after its last global write but thread 0's own.
-template <bool MUL>
+template <bool MUL, class TAB>
 __device__ __forceinline__ void rows_item(const TestDesc &T, int unit, double2 *xd, const double2 *yd, longlong2 *sm,
                                           ItemCtl &ctl) {
     // shared memory: two buffers of two rows, three for a product
@@ -264,11 +265,11 @@ __device__ __forceinline__ void rows_item(const TestDesc &T, int unit, double2 *
     const bool self = pr.x == pr.y;
     const unsigned odd = parity(pr.x) | parity(pr.y) << 1;  // of the lanes' rows
     int sx, sy;
-    longlong2 *X = rows_forward(T, pr, xd, sm, sm + 2 * C, odd, &ctl.top[0], &ctl.mag[0], &ctl.mid[0], sx);
+    longlong2 *X = rows_forward<TAB>(T, pr, xd, sm, sm + 2 * C, odd, &ctl.top[0], &ctl.mag[0], &ctl.mid[0], sx);
     longlong2 *other = X == sm ? sm + 2 * C : sm;
     longlong2 *Y = X;
     if constexpr (MUL) {
-        Y = rows_forward(T, pr, yd, other, sm + 4 * C, odd, &ctl.top[1], &ctl.mag[1], &ctl.mid[1], sy);
+        Y = rows_forward<TAB>(T, pr, yd, other, sm + 4 * C, odd, &ctl.top[1], &ctl.mag[1], &ctl.mid[1], sy);
         other = Y == other ? sm + 4 * C : other;
     } else {
         sy = sx;
@@ -290,7 +291,7 @@ __device__ __forceinline__ void rows_item(const TestDesc &T, int unit, double2 *
             ya = cshift(Y[ia], ny);
             yb = cshift(Y[ib], ny);
         }
-        split_pair<MUL>(a, b, __ldg(&swp[kc]), ya, yb);
+        split_pair<MUL>(a, b, TAB::load(&swp[kc]), ya, yb);
         X[ia] = a;
         if (!self) {
             X[ib] = b;
@@ -308,7 +309,7 @@ __device__ __forceinline__ void rows_item(const TestDesc &T, int unit, double2 *
     longlong2 *oa = x + (size_t)pr.x * C, *ob = x + (size_t)pr.y * C;
     mag = 0;
     int shift;
-    transform<1, true>(
+    transform<1, true, TAB>(
         pl, T.twr, other, X, odd, [&](int at, int, int) { return cshift(X[at], ns); },
         [&](longlong2 *, int, int e, int l, longlong2 v) {
             if (l && self) return;
@@ -341,52 +342,32 @@ __device__ __forceinline__ unsigned odd_columns(int g, int lg) {
     return 0x96u ^ (parity(g << lg) ? ~0u : 0u);  // 0..7 has 1, 2, 4 and 7 odd
 }
 
-// floor((hi) / k) for a signed 128-bit hi and 0 < k < 2^31, in 32-bit chunks
-__device__ __forceinline__ __int128 floor_div_small(__int128 hi, unsigned long long k) {
-    const bool neg = hi < 0;
-    unsigned __int128 a = neg ? (unsigned __int128)(-hi) : (unsigned __int128)hi;
-    unsigned __int128 q = 0;
-    unsigned long long rem = 0;
-#pragma unroll
-    for (int c = 3; c >= 0; c--) {
-        unsigned long long cur = (rem << 32) | (unsigned long long)((a >> (32 * c)) & 0xffffffffull);
-        q |= (unsigned __int128)(cur / k) << (32 * c);
-        rem = cur % k;
-    }
-    __int128 sq = (__int128)q;
-    if (neg) sq = rem ? -sq - 1 : -sq;
-    return sq;
+// x / k and its remainder for x < 2^64 and k_inv = floor((2^64 - 1) / k)
+__device__ __forceinline__ unsigned long long div_inv(unsigned long long x, unsigned long long k, unsigned long long k_inv,
+                                                      unsigned long long &rem) {
+    unsigned long long q = __umul64hi(x, k_inv);
+    rem = x - q * k;
+    for (; rem >= k; rem -= k) q++;  // at most twice
+    return q;
 }
-
-// Fold of the top region held in dig[top_t..L-1] plus the carry cy at 2^{s_L}
-// (reference src/ctx.c:345-375); returns the amount for digit 0.
-static __device__ __noinline__ long long fold_top(const TestDesc &T, long long *dig, long long cy) {
-    const int L = T.L, t = T.top_t;
-    __int128 H = (__int128)cy << T.top_shift;
-    int pos = 0;
-    for (int j = t; j < L; j++) {
-        H += (__int128)__ldcg(&dig[j]) << pos;
-        pos += T.bits[j];
+// floor(h / k) for a signed 128-bit h, in 32-bit digits of |h|; rem = h - k floor(h / k)
+__device__ __forceinline__ __int128 floor_div_inv(__int128 h, unsigned long long k, unsigned long long k_inv, __int128 &rem) {
+    const bool neg = h < 0;
+    const unsigned __int128 a = neg ? (unsigned __int128)(-h) : (unsigned __int128)h;
+    unsigned long long r = 0;
+    unsigned __int128 q = div_inv((unsigned long long)(a >> 64), k, k_inv, r);
+#pragma unroll
+    for (int c = 1; c >= 0; c--) {
+        const unsigned long long cur = (r << 32) | (unsigned)(a >> (32 * c));
+        q = (q << 32) | div_inv(cur, k, k_inv, r);
     }
-    const int m = T.top_m;
-    const __int128 K = (__int128)T.k;
-    __int128 lo = H & (((__int128)1 << m) - 1);
-    __int128 hi = H >> m;
-    __int128 q = floor_div_small(hi, T.k);
-    __int128 top = lo + ((hi - q * K) << m);
-    const __int128 span = K << m;
-    if (2 * top >= span) {
-        top -= span;
-        q += 1;
+    __int128 s = (__int128)q;
+    rem = (__int128)r;
+    if (neg) {
+        s = r ? -s - 1 : -s;
+        rem = r ? (__int128)(k - r) : 0;
     }
-    for (int j = t; j + 1 < L; j++) {
-        const int b = T.bits[j];
-        __int128 qq = (top + ((__int128)1 << (b - 1))) >> b;
-        dig[j] = (long long)(top - (qq << b));
-        top = qq;
-    }
-    if (t < L) dig[L - 1] = (long long)top;
-    return (long long)q;
+    return s;
 }
 
 // The 2G digit widths of the row segment starting at word j0, packed four to a word, in one
@@ -397,22 +378,22 @@ struct SegWidths {
     unsigned w[2 * G / 4];
 };
 
-template <int G>
+template <int G, class TAB>
 __device__ __forceinline__ SegWidths<G> load_segment_widths(const uint8_t *bits, int j0) {
     static_assert(G == 2 || G == 4 || G == 8, "column groups of 2, 4 or 8");
     SegWidths<G> s;
     if constexpr (G == 8) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(bits + j0));
+        const uint4 v = TAB::load(reinterpret_cast<const uint4 *>(bits + j0));
         s.w[0] = v.x;
         s.w[1] = v.y;
         s.w[2] = v.z;
         s.w[3] = v.w;
     } else if constexpr (G == 4) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(bits + j0));
+        const uint2 v = TAB::load(reinterpret_cast<const uint2 *>(bits + j0));
         s.w[0] = v.x;
         s.w[1] = v.y;
     } else {
-        s.w[0] = __ldg(reinterpret_cast<const unsigned *>(bits + j0));
+        s.w[0] = TAB::load(reinterpret_cast<const unsigned *>(bits + j0));
     }
     return s;
 }
@@ -420,6 +401,46 @@ __device__ __forceinline__ SegWidths<G> load_segment_widths(const uint8_t *bits,
 template <int G>
 __device__ __forceinline__ int seg_width(const SegWidths<G> &s, int i) {
     return (int)((s.w[i / 4] >> (8 * (i % 4))) & 0xffu);
+}
+
+// Fold of the top region (the last digits of the last segment) plus the carry cy at 2^{s_L}
+// (reference src/ctx.c:345-375); returns the amount for digit 0.  One thread of the whole test runs it
+// while the others wait, so it reads nothing back from memory and divides by k with its reciprocal.
+template <int G>
+__device__ __forceinline__ long long fold_segment(const TestDesc &T, const SegWidths<G> &bw, long long (&d)[2 * G],
+                                                  long long cy) {
+    const int first = 2 * G - (T.L - T.top_t);  // the top region's first digit in the segment
+    __int128 H = (__int128)cy << T.top_shift;
+    int pos = 0;
+#pragma unroll
+    for (int i = 0; i < 2 * G; i++)
+        if (i >= first) {
+            H += (__int128)d[i] << pos;
+            pos += seg_width(bw, i);
+        }
+    const int m = T.top_m;
+    const __int128 K = (__int128)T.k, span = K << m;
+    const __int128 lo = H & (((__int128)1 << m) - 1);
+    __int128 r;
+    __int128 q = floor_div_inv(H >> m, T.k, T.k_inv, r);
+    __int128 top = lo + (r << m);
+    if (2 * top >= span) {
+        top -= span;
+        q += 1;
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * G; i++)
+        if (i >= first) {
+            if (i == 2 * G - 1) {
+                d[i] = (long long)top;
+            } else {
+                const int b = seg_width(bw, i);
+                const __int128 c = (top + ((__int128)1 << (b - 1))) >> b;
+                d[i] = (long long)(top - (c << b));
+                top = c;
+            }
+        }
+    return (long long)q;
 }
 
 // v u 2^-(64 + n) rounded to the nearest integer; frac is the difference to it times 2^32.
@@ -445,7 +466,7 @@ __device__ __forceinline__ int col_scale(const FftPlan &pl, int e) {
     return 64 - max(3, pl.headroom) - e;
 }
 
-template <int G>
+template <int G, class TAB>
 __device__ __forceinline__ void segment_carries(const TestDesc &T, int g, const longlong2 *sm) {
     const int R = T.R, C = T.C;
     constexpr int LG = G == 8 ? 3 : G == 4 ? 2 : 1;
@@ -455,7 +476,7 @@ __device__ __forceinline__ void segment_carries(const TestDesc &T, int g, const 
     for (int r = threadIdx.x; r < R; r += blockDim.x) {
         const int j0 = 2 * (r * C + g * G);
         long long d[2 * G];
-        const SegWidths<G> bw = load_segment_widths<G>(T.bits, j0);
+        const SegWidths<G> bw = load_segment_widths<G, TAB>(T.bits, 2 * (r * T.pitch + g * G));
 #pragma unroll
         for (int l = 0; l < G; l++) {
             const longlong2 p = sm[turned<LG>(r, l)];
@@ -478,20 +499,18 @@ __device__ __forceinline__ void segment_carries(const TestDesc &T, int g, const 
             d[i] = v - (q << b);
             cy = q;
         }
+        const bool top = g == T.NG - 1 && r == R - 1;
+        if (top) cy = fold_segment<G>(T, bw, d, cy);
         longlong2 *dst = reinterpret_cast<longlong2 *>(T.dig + j0);  // j0 is even
 #pragma unroll
         for (int l = 0; l < G; l++) dst[l] = make_longlong2(d[2 * l], d[2 * l + 1]);
-        if (g == T.NG - 1 && r == R - 1) {
-            T.slot[0] = fold_top(T, T.dig, cy);  // this thread's own digits: visible
-        } else {
-            T.slot[g < T.NG - 1 ? (g + 1) * R + r : r + 1] = cy;
-        }
+        T.slot[top ? 0 : g < T.NG - 1 ? (g + 1) * R + r : r + 1] = cy;
     }
 }
 
 // One column group of one test, first half of the column pass.  Ends with a barrier after its
 // last global write.
-template <int LG>
+template <int LG, class TAB>
 __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int step, const double2 *xd, longlong2 *sm,
                                                  ItemCtl &ctl) {
     const bool track = step % T.err_every == 0;
@@ -507,16 +526,16 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
     int shift;
     const long long *osc = T.osc + 2 * (g << LG);
     unsigned err = 0, big = 0;
-    longlong2 *digits = transform<LG, true>(
+    longlong2 *digits = transform<LG, true, TAB>(
         pl, T.twc, sm, sm + (T.R << LG), odd,
         [&](int, int k, int l) {
             const int e = k * C + l;
-            return cmul(cshift(__ldcg(&x[e]), __ldcg(&rexp[k]) + se), conj_tw(__ldg(&t4[e])),
+            return cmul(cshift(__ldcg(&x[e]), __ldcg(&rexp[k]) + se), conj_tw(TAB::load(&t4[k * T.pitch + l])),
                         half_of(parity(k) ^ ((odd >> l) & 1)));
         },
         [&](longlong2 *dst, int, int r, int l, longlong2 v) {
             // unweight, scale and round
-            const longlong2 o = __ldg(reinterpret_cast<const longlong2 *>(osc + 2 * (r * C + l)));
+            const longlong2 o = TAB::load(reinterpret_cast<const longlong2 *>(osc + 2 * (r * T.pitch + l)));
             const int m = min((unsigned)(n + shift), 95u);
             int fx, fy;
             v.x = scale_round(v.x, o.x, m, fx);
@@ -527,7 +546,7 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
         },
         &ctl.mid[0], shift);
     const bool short_transform = n + shift < 0;  // the last place is above 1: too short for its data
-    segment_carries<1 << LG>(T, g, digits);
+    segment_carries<1 << LG, TAB>(T, g, digits);
     // |digit| >= 2^51 reports 0.5, as does a transform too short for its data
     if (!track) err = 0;
     if (big >= (1u << 19) || short_transform) err = 0x80000000u;
@@ -537,7 +556,7 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
     __syncthreads();
 }
 
-template <int G>
+template <int G, class TAB>
 __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool use_slots, int shift, longlong2 *sm) {
     const int R = T.R, C = T.C;
     constexpr int LG = G == 8 ? 3 : G == 4 ? 2 : 1;
@@ -553,7 +572,7 @@ __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool us
             d[2 * l + 1] = p.y;
         }
         long long cy = use_slots ? __ldcg(&T.slot[g * R + r]) : 0;
-        const SegWidths<G> bw = load_segment_widths<G>(T.bits, j0);
+        const SegWidths<G> bw = load_segment_widths<G, TAB>(T.bits, 2 * (r * T.pitch + g * G));
 #pragma unroll
         for (int i = 0; i < 2 * G - 1; i++) {
             if (cy) {
@@ -565,10 +584,10 @@ __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool us
             }
         }
         d[2 * G - 1] += cy;
-        const longlong2 *wv = reinterpret_cast<const longlong2 *>(T.w + j0);
+        const longlong2 *wv = reinterpret_cast<const longlong2 *>(T.w + 2 * (r * T.pitch + g * G));
 #pragma unroll
         for (int l = 0; l < G; l++) {
-            const longlong2 w = __ldg(wv + l);
+            const longlong2 w = TAB::load(wv + l);
             const long long a = shift_by(d[2 * l], shift), b = shift_by(d[2 * l + 1], shift);
             Acc x, y;
             x.mac(hi32(a), lo32(a), hi32(w.x), lo32(w.x));
@@ -581,7 +600,7 @@ __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool us
 // One column group of one test, second half of the column pass: absorb the carry-in, reweight,
 // forward column transform, twiddle.  `digit_bits` bounds the digits (T.digit_bits after a
 // product).  Ends with a barrier after its last global write.
-template <int LG>
+template <int LG, class TAB>
 __device__ __forceinline__ void col_forward_item(const TestDesc &T, int g, double2 *x, bool use_slots, int digit_bits,
                                                  longlong2 *sm, ItemCtl &ctl) {
     const int C = T.C;
@@ -590,25 +609,25 @@ __device__ __forceinline__ void col_forward_item(const TestDesc &T, int g, doubl
     if (g == 0 && threadIdx.x == 0) *T.emax = INT_MIN;
     // digits 2^shift w 2^-3: components below 2^59
     const int shift = 61 - digit_bits - max(0, pl.headroom - 3);
-    absorb_carries<1 << LG>(T, g, use_slots, shift, sm);
+    absorb_carries<1 << LG, TAB>(T, g, use_slots, shift, sm);
     __syncthreads();
     const unsigned odd = odd_columns(g, LG);
     int up;
     const int ex = pl.scale + 2 + 3 - shift;
     double2 *xg = x + (g << LG);
     const int4 *t4 = T.t4 + (g << LG);
-    transform<LG, false>(
+    transform<LG, false, TAB>(
         pl, T.twc, sm + (T.R << LG), sm, odd, [&](int, int r, int l) { return sm[turned<LG>(r, l)]; },
         [&](longlong2 *, int, int k, int l, longlong2 v) {
             const int e = k * C + l;
-            const longlong2 z = cmul(v, __ldg(&t4[e]), half_of(parity(k) ^ ((odd >> l) & 1)));
+            const longlong2 z = cmul(v, TAB::load(&t4[k * T.pitch + l]), half_of(parity(k) ^ ((odd >> l) & 1)));
             xg[e] = make_double2(from_fixed(z.x, ex - up), from_fixed(z.y, ex - up));
         },
         &ctl.mid[0], up);
 }
 
 // One column group of one test: its digits.  Ends with a barrier.
-template <int LG>
+template <int LG, class TAB>
 __device__ __forceinline__ void col_digits_item(const TestDesc &T, int g, const double2 *xd, long long *dig,
                                                 longlong2 *sm, ItemCtl &ctl) {
     const int C = T.C, R = T.R;
@@ -628,11 +647,11 @@ __device__ __forceinline__ void col_digits_item(const TestDesc &T, int g, const 
     const int n = se - 4 - pl.scale - T.idig_exp;
     const unsigned odd = odd_columns(g, LG);
     int shift;
-    transform<LG, true>(
+    transform<LG, true, TAB>(
         pl, T.twc, sm + (R << LG), sm, odd,
         [&](int at, int k, int l) {
             const longlong2 d = sm[at];
-            return cmul(make_longlong2(to_fixed(d.x, se), to_fixed(d.y, se)), conj_tw(__ldg(&t4[k * C + l])),
+            return cmul(make_longlong2(to_fixed(d.x, se), to_fixed(d.y, se)), conj_tw(TAB::load(&t4[k * T.pitch + l])),
                         half_of(parity(k) ^ ((odd >> l) & 1)));
         },
         [&](longlong2 *, int, int r, int l, longlong2 v) {

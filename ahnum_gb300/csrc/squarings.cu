@@ -81,11 +81,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_squarings(const TestDe
         const int step = step0 + (int)st;
         if (step < T.count) {
             if (r < nr)
-                rows_item<false>(T, it.unit, T.x, nullptr, sm, s_ctl);
+                rows_item<false, GlobalTables>(T, it.unit, T.x, nullptr, sm, s_ctl);
             else if (r < nr + nc)
-                col_inverse_item<LG>(T, it.unit, step, T.x, sm, s_ctl);
+                col_inverse_item<LG, GlobalTables>(T, it.unit, step, T.x, sm, s_ctl);
             else
-                col_forward_item<LG>(T, it.unit, T.x, true, T.digit_bits, sm, s_ctl);
+                col_forward_item<LG, GlobalTables>(T, it.unit, T.x, true, T.digit_bits, sm, s_ctl);
         }
         // each item ends with a barrier after its last global write (but for thread 0's own):
         // publish them, then count
