@@ -24,9 +24,8 @@ bool kc_ok(kc_engine *e, cudaError_t rc) {
 }
 
 int kc_get_limbs(kc_engine *e, const double *x, uint64_t *limbs) {
-    std::vector<int64_t> d(e->lay.L);
-    if (kc_to_digits(e, x, d.data())) return e->err ? e->err : -1;
-    e->lay.digits_to_limbs(d.data(), limbs);
+    if (kc_fetch_digits(e, x)) return e->err ? e->err : -1;
+    e->lay.digits_to_limbs(reinterpret_cast<const int64_t *>(e->h_dig), limbs);
     return 0;
 }
 
@@ -358,6 +357,17 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
     return e;
 }
 
+// the digits of x into the pinned staging buffer e->h_dig; waits
+int kc_fetch_digits(kc_engine *e, const double *x) {
+    DeviceGuard dg(e->device);
+    launch_col_digits(e->ls, (const double2 *)x);
+    if (!check_launch(e)) return e->err;
+    if (!ok(e, cudaMemcpyAsync(e->h_dig, e->d_dig, e->lay.L * sizeof(long long), cudaMemcpyDeviceToHost, e->stream)) ||
+        !wait_queue(e))
+        return e->err;
+    return 0;
+}
+
 extern "C" {
 
 void kc_engine_free(kc_engine *e) {
@@ -403,14 +413,8 @@ int kc_from_digits(kc_engine *e, double *x, const int64_t *digits) {
 }
 
 int kc_to_digits(kc_engine *e, const double *x, int64_t *digits) {
-    DeviceGuard dg(e->device);
-    const size_t L = e->lay.L;
-    launch_col_digits(e->ls, (const double2 *)x);
-    if (!check_launch(e)) return e->err;
-    if (!ok(e, cudaMemcpyAsync(e->h_dig, e->d_dig, L * sizeof(long long), cudaMemcpyDeviceToHost, e->stream)) ||
-        !wait_queue(e))
-        return e->err;
-    std::memcpy(digits, e->h_dig, L * sizeof(long long));
+    if (kc_fetch_digits(e, x)) return e->err;
+    std::memcpy(digits, e->h_dig, e->lay.L * sizeof(long long));
     return 0;
 }
 

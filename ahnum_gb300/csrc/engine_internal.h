@@ -53,6 +53,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
 
 // helpers shared with the batch engine (engine.cu)
 bool kc_ok(kc_engine *e, cudaError_t rc);
+int kc_fetch_digits(kc_engine *e, const double *x);  // into the pinned e->h_dig; waits
 int kc_get_limbs(kc_engine *e, const double *x, uint64_t *limbs);   // canonical, waits
 int kc_set_limbs(kc_engine *e, double *x, const uint64_t *limbs);
 int kc_mul_small_host(kc_engine *e, double *x, int64_t m);

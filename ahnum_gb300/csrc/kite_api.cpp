@@ -10,6 +10,7 @@
 #include "../../include/kite.h"
 #include "../../include/kite_cuda.h"
 #include "../../include/kite_ntt.h"
+#include "engine_internal.h"
 #include "kite_internal.h"
 
 using kg::Layout;
@@ -191,12 +192,7 @@ void kite_get_limbs(kite_ctx *ctx, const kite_num *x, uint64_t *limbs) {
         if (kn_get_limbs(ctx->ntt, wd(x), limbs)) std::memset(limbs, 0, ctx->lay.nlimbs * sizeof(uint64_t));
         return;
     }
-    int64_t *d = ctx->dig.data();
-    if (kc_to_digits(ctx->eng, fp(x), d)) {
-        std::memset(limbs, 0, ctx->lay.nlimbs * sizeof(uint64_t));
-        return;
-    }
-    ctx->lay.digits_to_limbs(d, limbs);
+    if (kc_get_limbs(ctx->eng, fp(x), limbs)) std::memset(limbs, 0, ctx->lay.nlimbs * sizeof(uint64_t));
 }
 
 void kite_set_limbs(kite_ctx *ctx, kite_num *x, const uint64_t *limbs) {

@@ -52,7 +52,6 @@ struct Layout {
 
   private:
     int64_t fold_top(int64_t *d, int64_t cy) const;
-    void reduce_mod_N(uint64_t *a, size_t na) const;
 };
 
 // y = base^(N+1) mod N (nl limbs) -> base^(N-1) mod N, also when gcd(base, N) > 1.
