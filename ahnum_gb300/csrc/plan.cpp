@@ -8,6 +8,7 @@
 #include <cstdlib>
 
 #include "../../include/kite_cuda.h"
+#include "kernels.h"
 
 #include <algorithm>
 #include <cmath>
@@ -102,12 +103,40 @@ bool choose_shape(uint32_t H, uint32_t &R, uint32_t &C) {
     return R != 0;
 }
 
-static int radix_stages(uint32_t n) {
-    int st = 0;
-    for (; n % 4 == 0; n /= 4) st++;
-    for (uint32_t p : {2u, 3u, 5u, 7u})
-        for (; n % p == 0; n /= p) st++;
-    return st;
+// Rounds of a CTA in the stages of `count` transforms of length n together, in units of a radix-4
+// round: a stage whose butterflies do not fill the CTA costs as much as one that does.
+static double stage_rounds(uint32_t n, uint32_t count) {
+    static const std::pair<uint32_t, double> radix[] = {{4, 1.0}, {2, 0.5}, {3, 0.9}, {5, 1.9}, {7, 3.0}};
+    double sum = 0;
+    uint32_t m = n;
+    for (const auto &[p, weight] : radix)
+        for (; m % p == 0; m /= p) sum += weight * ((count * (n / p) + kThreads - 1) / kThreads);
+    return sum;
+}
+
+// Predicted time in us of one squaring of a chain (chain.cu) of R x C in column groups of G, from
+// what every CTA does in a row: fitted to 310 shapes of 21 lengths from 512 to 1769472 digits.
+//  - a fixed part, mostly the three grid barriers and the first loads after them;
+//  - the rounds of a row pair's and a column group's stages, there and back, and the rounds over their
+//    points besides (loads, squares, carries; a column group has two such passes);
+//  - 1.6 times that in a wave which puts two CTAs on an SM: alone, a CTA waits for its own latencies;
+//  - a wave more wherever a pass has more items than CTAs stay: one per SM, or two up to kTwoCtaSmem;
+//  - the tables read from L2 when they do not stay in shared memory.
+static double chain_us(uint32_t R, uint32_t C, int G, int nsm) {
+    constexpr size_t kTwoCtaSmem = 108 * 1024;
+    const uint32_t pairs = R / 2 + 1, groups = C / G, most = std::max(pairs, groups);
+    const size_t smem = 16 * std::max((size_t)4 * C, (size_t)2 * R * G);
+    const size_t table = 16 * ((size_t)2 * C + R + (size_t)3 * R * G) + (size_t)2 * R * G;
+    const bool keeps = most <= (uint32_t)nsm && smem + table <= kMaxChainSmem;
+    const uint32_t resident = std::min<uint32_t>(most, nsm * (!keeps && smem <= kTwoCtaSmem ? 2 : 1));
+    const auto pass = [&](uint32_t items, uint32_t n, uint32_t count, double passes) {
+        double us = -2.16 * passes;
+        const double once = 0.475 * 2 * stage_rounds(n, count) + 0.54 * passes * ((count * n + kThreads - 1) / kThreads);
+        for (uint32_t left = items; left; left -= std::min(left, resident))
+            us += 2.16 * passes + once * (std::min(left, resident) > (uint32_t)nsm ? 1.6 : 1.0);
+        return us;
+    };
+    return 6.75 + pass(pairs, C, 2, 1) + pass(groups, R, G, 2) + (keeps ? 0 : 3.1) + 0.18 * std::log2((double)R);
 }
 
 // Latency shapes chosen by the autotuner (or a tuning file), by FFT length L = 2H: (R, G).
@@ -145,8 +174,6 @@ bool choose_latency_shape(uint32_t H, int nsm, unsigned min_bits, unsigned top_d
             return true;
         }
     }
-    // FP64 lane-operations per point of each pass (measured: rows ~53, each column pass ~24),
-    // a fixed cost per stage barrier, and the load of the busiest SM.
     double best = 1e300;
     R = C = 0;
     G = kGroup;
@@ -156,10 +183,7 @@ bool choose_latency_shape(uint32_t H, int nsm, unsigned min_bits, unsigned top_d
         const uint32_t r = H / c;
         for (int g : {2, 4, 8}) {
             if (!group_fits(g, min_bits, top_digits)) continue;
-            const double pairs = r / 2 + 1, groups = c / g;
-            const double rows = std::ceil(pairs / nsm) * 106.0 * c + 800.0 * (2 * radix_stages(c) + 2);
-            const double cols = std::ceil(groups / nsm) * 24.0 * r * g + 800.0 * (radix_stages(r) + 2);
-            const double cost = rows + 2 * cols;
+            const double cost = chain_us(r, c, g, nsm) + (r < 4 ? 1e3 : 0);  // two rows: where nothing else fits
             if (cost < best - 1e-9) {
                 best = cost;
                 R = r;
