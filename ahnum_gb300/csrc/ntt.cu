@@ -1,6 +1,6 @@
 // Exact integer-NTT squaring modulo N = k*2^n - 1 (include/kite_ntt.h).
 //
-// One modular squaring is four kernels over a test's W words of w bits:
+// One modular squaring is three or four kernels over a test's W words of w bits:
 //   kn_col_fwd   per group of G columns of the R x C four-step layout: words -> residues modulo
 //                four primes, forward column NTT (decimation in frequency, natural order in,
 //                bit-reversed out), times the four-step twiddle w_NP^(k_r c).
@@ -13,6 +13,8 @@
 //   kn_reduce    per test, one block: the segment carries into the words of P = x^2, Montgomery
 //                reduction P 2^-n == B + k A (mod N) for P = A + B 2^n, A < 2^n, plus an
 //                optional constant, carry, and the top fold T 2^n == q + r 2^n for T = q k + r.
+//                Only after the last squaring of a chain: before, kn_col_fwd takes its words from the
+//                product itself (Fold).
 // Reference: gpu/ntt_reg.metal:90-246 (the four-step NTT passes), gpu/sq.metal:23-192 (residues,
 // Garner CRT, carry, REDC, fold), gpu/gpu_ctx.h:57-322 (tables and the pass sequence).
 //
@@ -25,6 +27,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -177,17 +180,132 @@ __device__ __forceinline__ int col_addr(int i, int rp_len, int e, int l) {
     return ((i * rp_len + e + (e >> clog2<B>())) << 3) + l;
 }
 
-template <int A, int B>
-__device__ __forceinline__ void col_fwd_item(uint32_t *sm, const Desc &D, int g, const uint64_t *src, uint32_t *dst) {
+// The reduction inside the next squaring's column pass.  E = B + k A (+ c) for the product
+// P = A + B 2^n needs no carry beyond two words when the words may be redundant: with the segments'
+// carries added where they belong, e_j < 2^(w+33); one word takes e_j mod 2^w, the next one
+// e_j >> w, and what that leaves above w bits (0 or 1) goes one word further.  The words are then at
+// most 2^w instead of 2^w - 1, which the primes have to allow (NumLayout::lazy), and the value is
+// exactly E.  Every CTA computes its own eight columns' words from the product, so nothing waits for
+// one block that walks through the whole number: that took 16 of the 41 us of a squaring at n = 369717,
+// now 20.4 us together with launches that overlap; 64 tests of n = 300000 to 700000 130 -> 101 us.
+struct Fold {
+    uint64_t q, lo, r0, r1;  // T = E >> n = q k + r: q joins word 0, r 2^n the words WN0 and WN0 + 1
+};
+
+__device__ __forceinline__ uint64_t product_word(const Desc &D, uint32_t j) {
+    uint64_t v = D.pw[j];
+    if ((j & 7) < 2 && j >= 8) {
+        const ulonglong2 c = D.seg[(j >> 3) - 1];  // < 2^(w+20): its low word and the rest
+        v += (j & 7) == 0 ? c.x & ((1ull << D.w) - 1) : (c.x >> D.w) | (c.y << (64 - D.w));
+    }
+    return v;
+}
+
+__device__ __forceinline__ u128 reduced_word(const Desc &D, int j, const uint64_t *addend) {
+    if (j < 0 || j > (int)D.W) return 0;
+    const uint64_t low = (1ull << D.BN0) - 1;
+    const uint32_t s = D.WN0 + j;
+    const uint64_t v0 = s < D.NP ? product_word(D, s) : 0, v1 = D.BN0 && s + 1 < D.NP ? product_word(D, s + 1) : 0;
+    const uint64_t a = j < (int)D.WN0 ? product_word(D, j) : j == (int)D.WN0 ? product_word(D, j) & low : 0;
+    u128 e = (u128)D.k * a + (v0 >> D.BN0) + ((v1 & low) << (D.w - D.BN0));
+    if (addend && j < (int)D.W) e += addend[j];
+    return e;
+}
+
+// Two steps of carries among WIDTH lanes that hold consecutive words; lanes 0 and 1 take theirs from
+// (c1, c1p, c2): e's carry of the word before, and the single bits that it leaves.
+__device__ __forceinline__ uint64_t two_carries(u128 e, uint32_t w, int lane, int width, uint32_t c1_before, uint32_t c2_before,
+                                                uint32_t *c1_out, uint32_t *c2_out) {
+    const uint64_t M = (1ull << w) - 1;
+    const uint32_t c1 = (uint32_t)(e >> w);
+    uint32_t in = __shfl_up_sync(0xffffffffu, c1, 1, width);
+    const uint64_t x = ((uint64_t)e & M) + (lane ? in : c1_before);
+    const uint32_t c2 = (uint32_t)(x >> w);
+    in = __shfl_up_sync(0xffffffffu, c2, 1, width);
+    *c1_out = c1;
+    *c2_out = c2;
+    return (x & M) + (lane ? in : c2_before);
+}
+
+// One warp: T = E >> n from the words WN0 .. W of E, its quotient and remainder by k.
+__device__ __forceinline__ void fold_of(const Desc &D, const uint64_t *addend, Fold *f) {
+    const int lane = threadIdx.x & 31;
+    uint32_t c1, c2;
+    const u128 e = reduced_word(D, (int)D.WN0 - 2 + lane, addend);
+    const uint64_t x = two_carries(e, D.w, lane, 32, 0, 0, &c1, &c2);  // exact from lane 2 on: word WN0
+    const uint64_t xn = __shfl_sync(0xffffffffu, x, 2);
+    u128 T = xn >> D.BN0;
+    int bad = 0;
+    uint32_t sh = D.w - D.BN0;
+    for (uint32_t j = D.WN0 + 1; j <= D.W; j++, sh += D.w) {
+        const uint64_t v = __shfl_sync(0xffffffffu, x, (int)(j - D.WN0) + 2);
+        if (!v) continue;
+        if (j == D.W) bad |= 2;
+        else if (sh >= 128 || (sh > 64 && (v >> (128 - sh)) != 0)) bad |= 4;
+        else T += (u128)v << sh;
+    }
+    if (lane == 0) {
+        const ulonglong2 out = D.seg[(D.NP >> 3) - 1];
+        if (out.x | out.y) bad |= 1;
+        uint64_t q, r0;
+        if ((T >> 64) == 0) {  // always for k < 2^30 and a number below N: T < 2^(2 log2 k + 3)
+            const uint64_t t64 = (uint64_t)T;
+            q = t64 / D.k;
+            r0 = t64 - q * D.k;
+        } else {
+            const u128 qq = T / D.k;
+            if (qq >> (D.w + 30)) bad |= 4;
+            q = (uint64_t)qq;
+            r0 = (uint64_t)(T - qq * D.k);
+        }
+        const u128 r = (u128)r0 << D.BN0;
+        f->q = q;
+        f->lo = xn & ((1ull << D.BN0) - 1);
+        f->r0 = (uint64_t)r & ((1ull << D.w) - 1);
+        f->r1 = (uint64_t)(r >> D.w);
+        if (f->r1 && D.WN0 + 1 >= D.W) bad |= 8;
+        if (bad) atomicOr(D.status, bad);
+    }
+}
+
+// Word j = r C + 8 g + l of E, by lane l of the eight that hold the row.
+__device__ __forceinline__ uint64_t folded_word(const Desc &D, int j, int l, const uint64_t *addend, const Fold &f) {
+    u128 e = reduced_word(D, j, addend);
+    if (j == 0) e += f.q;
+    // the two words before the eight: lanes 6 and 7 evaluate them besides their own
+    const u128 h = l >= 6 ? reduced_word(D, j - 8, addend) : 0;
+    uint32_t c1, c2, h1, h2;
+    (void)two_carries(h, D.w, l, 8, 0, 0, &h1, &h2);
+    const uint32_t c1b = __shfl_sync(0xffffffffu, h1, 7, 8), c2b = __shfl_sync(0xffffffffu, h2, 7, 8);
+    uint64_t x = two_carries(e, D.w, l, 8, c1b, c2b, &c1, &c2);
+    if (j >= (int)D.W) x = 0;  // its CTA may not hold the fold
+    else if (j == (int)D.WN0) x = f.lo + f.r0;
+    else if (j == (int)D.WN0 + 1) x = f.r1;
+    else if (j > (int)D.WN0) x = 0;
+    return x;
+}
+
+template <int A, int B, bool FOLD>
+__device__ __forceinline__ void col_fwd_item(uint32_t *sm, const Desc &D, int g, const uint64_t *src, uint32_t *dst, Fold &f) {
     constexpr int R = A * B, RP = R + R / B;
     const int C = (int)D.C;
     const int np = (int)D.np;
+    if (FOLD) {  // src: the constant to add
+        bool mine = g == 0;
+        for (uint32_t j = D.WN0; j < D.W; j++) mine |= (int)((j & (C - 1)) >> 3) == g;
+        if (mine) {
+            if (threadIdx.x < 32) fold_of(D, src, &f);
+            __syncthreads();
+        }
+    }
     // NP >= 2W: the words at r C + c >= W, hence every row r >= R/2, are the product's zero
     // padding; only the lower half is converted and stored
     for (int e = threadIdx.x; e < (R / 2) * kG; e += blockDim.x) {
         const int r = e >> 3, l = e & 7;
         const uint32_t j = (uint32_t)r * C + g * kG + l;
-        const uint64_t word = j < D.W ? src[j] : 0;
+        uint64_t word;
+        if (FOLD) word = folded_word(D, (int)j, l, src, f);  // whole warps: (R / 2) * kG is a multiple of 32
+        else word = j < D.W ? src[j] : 0;
         for (int i = 0; i < np; i++) sm[col_addr<B>(i, RP, r, l)] = residue(word, D.pr[i]);
     }
     __syncthreads();
@@ -217,24 +335,56 @@ __device__ __forceinline__ void col_fwd_item(uint32_t *sm, const Desc &D, int g,
     __syncthreads();
 }
 
-// src overrides the test's operand (x, or y for the second operand of a product)
+// The descriptor of the item's test, in shared memory: its fields are read between dependent loads.
+__device__ __forceinline__ void stage_desc(Desc *d, int *held, const Desc *descs, int test) {
+    static_assert(sizeof(Desc) % 8 == 0, "copied by 8-byte words");
+    if (*held == test) return;  // uniform: thread 0 wrote it before a barrier
+    __syncthreads();
+    const uint64_t *from = reinterpret_cast<const uint64_t *>(descs + test);
+    for (int i = threadIdx.x; i < (int)(sizeof(Desc) / 8); i += blockDim.x) reinterpret_cast<uint64_t *>(d)[i] = from[i];
+    if (threadIdx.x == 0) *held = test;
+    __syncthreads();
+}
+
+// Programmatic dependent launch: what a kernel reads before pdl_enter no kernel writes.
+__device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_leave() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A kernel's start: the first item's descriptor while the previous kernel still runs.  Lists and
+// descriptors are written by copies, which no kernel overtakes.
+__device__ __forceinline__ void first_desc(Desc *d, int *held, const Desc *descs, const int2 *items, int nitems) {
+    if (threadIdx.x == 0) *held = -1;
+    __syncthreads();
+    if ((int)blockIdx.x < nitems) stage_desc(d, held, descs, items[blockIdx.x].x);
+    pdl_enter();
+    pdl_leave();
+}
+
+// src overrides the test's operand (x, or y for the second operand of a product); with FOLD the
+// words come from the last product's reduction, and src is the constant to add
+template <bool FOLD>
 __global__ void __launch_bounds__(kColThreads) kn_col_fwd(const Desc *descs, const int2 *items, int nitems,
                                                           int second, const uint64_t *src_o) {
     extern __shared__ uint32_t sm[];
+    __shared__ Desc s_desc;
+    __shared__ Fold s_fold;
+    __shared__ int s_held;
+    first_desc(&s_desc, &s_held, descs, items, nitems);
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 wi = items[it];
-        const Desc &D = descs[wi.x];
-        const uint64_t *src = src_o ? src_o : (second ? D.y : D.x);
+        stage_desc(&s_desc, &s_held, descs, wi.x);
+        const Desc &D = s_desc;
+        const uint64_t *src = FOLD ? (src_o ? src_o : D.addend) : src_o ? src_o : (second ? D.y : D.x);
         uint32_t *dst = second ? D.res2 : D.res;
         switch (log2i(D.R)) {
-        case 3: col_fwd_item<2, 4>(sm, D, wi.y, src, dst); break;
-        case 4: col_fwd_item<4, 4>(sm, D, wi.y, src, dst); break;
-        case 5: col_fwd_item<4, 8>(sm, D, wi.y, src, dst); break;
-        case 6: col_fwd_item<8, 8>(sm, D, wi.y, src, dst); break;
-        case 7: col_fwd_item<8, 16>(sm, D, wi.y, src, dst); break;
-        case 8: col_fwd_item<16, 16>(sm, D, wi.y, src, dst); break;
-        case 9: col_fwd_item<16, 32>(sm, D, wi.y, src, dst); break;
-        default: col_fwd_item<32, 32>(sm, D, wi.y, src, dst); break;
+        case 3: col_fwd_item<2, 4, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
+        case 4: col_fwd_item<4, 4, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
+        case 5: col_fwd_item<4, 8, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
+        case 6: col_fwd_item<8, 8, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
+        case 7: col_fwd_item<8, 16, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
+        case 8: col_fwd_item<16, 16, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
+        case 9: col_fwd_item<16, 32, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
+        default: col_fwd_item<32, 32, FOLD>(sm, D, wi.y, src, dst, s_fold); break;
         }
     }
 }
@@ -303,9 +453,13 @@ __device__ __forceinline__ void row_item(uint32_t *sm, const Desc &D, int pos) {
 template <bool MUL>
 __global__ void __launch_bounds__(kRowThreads) kn_rows(const Desc *descs, const int2 *items, int nitems) {
     extern __shared__ uint32_t sm[];
+    __shared__ Desc s_desc;
+    __shared__ int s_held;
+    first_desc(&s_desc, &s_held, descs, items, nitems);
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 wi = items[it];
-        const Desc &D = descs[wi.x];
+        stage_desc(&s_desc, &s_held, descs, wi.x);
+        const Desc &D = s_desc;
         switch (log2i(D.C)) {
         case 3: row_item<2, 4, MUL>(sm, D, wi.y); break;
         case 4: row_item<4, 4, MUL>(sm, D, wi.y); break;
@@ -415,9 +569,13 @@ __device__ __forceinline__ void col_inv_item(uint32_t *sm, const Desc &D, int g)
 
 __global__ void __launch_bounds__(kColThreads) kn_col_inv(const Desc *descs, const int2 *items, int nitems) {
     extern __shared__ uint32_t sm[];
+    __shared__ Desc s_desc;
+    __shared__ int s_held;
+    first_desc(&s_desc, &s_held, descs, items, nitems);
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const int2 wi = items[it];
-        const Desc &D = descs[wi.x];
+        stage_desc(&s_desc, &s_held, descs, wi.x);
+        const Desc &D = s_desc;
         switch (log2i(D.R)) {
         case 3: col_inv_item<2, 4>(sm, D, wi.y); break;
         case 4: col_inv_item<4, 4>(sm, D, wi.y); break;
@@ -464,12 +622,16 @@ __device__ u128 resolve_chunks(uint64_t *v, uint32_t len, uint32_t S, uint32_t w
     return *top;
 }
 
-// x_o, add_o override the test's result array and addend
+// x_o, add_o override the test's result array and addend.  With NUMBER the product is the W words at
+// num, normalised: its reduction num 2^-n takes a number out of the Montgomery form.
+template <bool NUMBER>
 __global__ void __launch_bounds__(kReduceThreads) kn_reduce(const Desc *descs, const int *tests, uint64_t *x_o,
-                                                            const uint64_t *add_o) {
+                                                            const uint64_t *add_o, const uint64_t *num) {
     __shared__ u128 co[kReduceThreads];
     __shared__ u128 top;
     const Desc &D = descs[tests[blockIdx.x]];
+    pdl_enter();
+    pdl_leave();
     uint64_t *X = x_o ? x_o : D.x;
     const uint64_t *addend = x_o ? add_o : D.addend;
     const int t = threadIdx.x, T = blockDim.x;
@@ -477,15 +639,15 @@ __global__ void __launch_bounds__(kReduceThreads) kn_reduce(const Desc *descs, c
     const uint64_t M = (1ull << w) - 1;
     // The descriptor's fields are read once: the stores below go through global pointers the
     // compiler cannot tell apart from the descriptor.
-    const uint32_t NP = D.NP, Wn = D.W, WN0 = D.WN0, BN0 = D.BN0;
+    const uint32_t Wn = D.W, NP = NUMBER ? Wn : D.NP, WN0 = D.WN0, BN0 = D.BN0;
     const uint64_t kk = D.k;
     const ulonglong2 *__restrict__ seg = D.seg;
-    uint64_t *__restrict__ pw = D.pw;
+    uint64_t *__restrict__ pw = NUMBER ? const_cast<uint64_t *>(num) : D.pw;
     int *status = D.status;
     constexpr int U = 8;  // loads in flight per thread
     // 1. product words: the transform kernels left P as 8-word segments, each normalised, with
     //    the carry out of segment s in seg[s]; add every segment's carry into the next one
-    {
+    if (!NUMBER) {
         const uint32_t nseg = NP >> 3, per = (nseg + T - 1) / T;
         const uint32_t s0 = (uint32_t)t * per, s1 = min(nseg, s0 + per);
         ulonglong2 *__restrict__ pw2 = reinterpret_cast<ulonglong2 *>(pw);
@@ -603,6 +765,22 @@ __global__ void __launch_bounds__(kReduceThreads) kn_reduce(const Desc *descs, c
     }
 }
 
+// The words X (below 2^w each) as 64-bit limbs, and the status word after the last one.
+__global__ void kn_limbs(const uint64_t *X, uint32_t W, uint32_t w, uint64_t *limbs, uint32_t nlimbs, const int *status) {
+    pdl_enter();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > nlimbs) return;
+    if (i == nlimbs) {
+        limbs[i] = (uint64_t)(int64_t)*status;
+        return;
+    }
+    const uint64_t bit = 64ull * i;
+    uint32_t j = (uint32_t)(bit / w), have = w - (uint32_t)(bit % w);
+    uint64_t v = j < W ? X[j] >> (w - have) : 0;
+    for (j++; have < 64 && j < W; j++, have += w) v |= X[j] << have;
+    limbs[i] = v;
+}
+
 // ---- host tables ------------------------------------------------------------------------------
 
 uint32_t mulmod(uint32_t a, uint32_t b, uint32_t p) { return (uint32_t)((uint64_t)a * b % p); }
@@ -656,6 +834,32 @@ size_t padded_len(uint32_t n) {
 }
 size_t col_smem_bytes(uint32_t R) { return (size_t)kPrimes * padded_len(R) * kG * 4; }
 size_t row_smem_bytes(uint32_t C) { return (size_t)kPrimes * padded_len(C) * 4; }
+
+// Kernels of one stream launch with programmatic stream serialization (each enters through pdl_enter),
+// so the next one's CTAs are scheduled, and read their descriptors, while this one drains; the first of
+// a call is launched plainly, and so is every one with KITE_GB300_PDL=0.
+bool pdl_enabled() {
+    static const bool on = [] {
+        const char *p = std::getenv("KITE_GB300_PDL");
+        return !(p && p[0] == '0');
+    }();
+    return on;
+}
+
+template <class... P, class... A>
+void launch(bool overlap, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = overlap && pdl_enabled() ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 struct Plan {
     uint32_t NP = 0, R = 0, C = 0;
@@ -772,6 +976,7 @@ void sub_in(std::vector<uint64_t> &a, const std::vector<uint64_t> &b) {
 struct NumLayout {
     uint64_t k = 0, n = 0;
     uint32_t np = 0, W = 0, w = 0, NP = 0;
+    bool lazy = false;  // words of up to 2^w may be squared (Fold)
     size_t nlimbs = 0;
     std::vector<uint64_t> N;  // modulus, nlimbs limbs
     bool build(uint64_t k, uint64_t n);
@@ -794,6 +999,8 @@ struct kn_engine : kn::NumLayout {
     ulonglong2 *d_seg = nullptr;
     uint64_t *d_pw = nullptr;
     uint64_t *d_addend = nullptr;
+    uint64_t *d_out = nullptr;  // W words, then the limbs and the status of the number being read
+    std::mutex out_mu;          // held from the first write to d_out until it is copied
     int64_t addend_c = 0;
     bool addend_ok = false;
     int err = 0;
@@ -965,7 +1172,8 @@ bool prepare_smem(int device, size_t col_smem, size_t row_smem) {
     std::lock_guard<std::mutex> lock(mu);
     bool ok = true;
     if (col_smem > col_hw[device]) {
-        ok = ok && cudaFuncSetAttribute(kn_col_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(kn_col_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(kn_col_fwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(kn_col_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem) == cudaSuccess;
         if (ok) col_hw[device] = col_smem;
     }
@@ -1002,6 +1210,12 @@ bool kn::NumLayout::build(uint64_t kk, uint64_t nn) {
     choose_sizes(k, n, np, w, W, NP);
     if (!NP || NP > (1u << 20)) return false;
     nlimbs = (size_t)((n + 64 + 63) / 64);
+    // the coefficients of words up to 2^w still lie below the product of the primes (at w = 50, 4
+    // primes always; elsewhere all but the last few word counts before a smaller w), a carry fits 32
+    // bits, and word 0's part of the fold stays clear of the top words
+    u128 prod = 1;
+    for (uint32_t i = 0; i < np; i++) prod *= kP[i];
+    lazy = ((u128)W << (2 * w)) < prod && w >= 33 && n / w >= 8;
     N = modulus(k, n, nlimbs);
     return true;
 }
@@ -1057,6 +1271,7 @@ kn_engine *kn_engine_new(uint64_t k, uint64_t n, int device) {
               kok(e, cudaMalloc((void **)&e->d_seg, (size_t)(NP / kG) * sizeof(ulonglong2))) &&
               kok(e, cudaMalloc((void **)&e->d_pw, (size_t)NP * 8)) &&
               kok(e, cudaMalloc((void **)&e->d_addend, (size_t)e->W * 8)) &&
+              kok(e, cudaMalloc((void **)&e->d_out, ((size_t)e->W + e->nlimbs + 1) * 8)) &&
               kok(e, cudaMalloc((void **)&e->d_status, sizeof(int))) &&
               kok(e, cudaMalloc((void **)&e->d_cols, (C / kG) * sizeof(int2))) &&
               kok(e, cudaMalloc((void **)&e->d_rows, R * sizeof(int2))) &&
@@ -1120,7 +1335,7 @@ void kn_engine_free(kn_engine *e) {
     cudaSetDevice(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
     for (void *p : {(void *)e->d_desc, (void *)e->d_res, (void *)e->d_res2, (void *)e->d_seg, (void *)e->d_pw,
-                    (void *)e->d_addend, (void *)e->d_status, (void *)e->d_cols, (void *)e->d_rows, (void *)e->d_test})
+                    (void *)e->d_addend, (void *)e->d_out, (void *)e->d_status, (void *)e->d_cols, (void *)e->d_rows, (void *)e->d_test})
         if (p) cudaFree(p);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
@@ -1161,45 +1376,67 @@ int kn_set_limbs(kn_engine *e, uint64_t *x, const uint64_t *limbs) {
     return kok(e, cudaStreamSynchronize(e->stream)) ? 0 : -1;
 }
 
+// x~ 2^-n mod N by the product's reduction and the repacking on the GPU; a value of N or more (a
+// number equal to N, or one that was never reduced) is finished on the host.  On GB300, n = 300000 to
+// 700000: 55 us a number, half of it the reduction's one block; 112 us with the arithmetic on the host.
 int kn_get_limbs(kn_engine *e, const uint64_t *x, uint64_t *limbs) {
     if (!e || e->err) return -1;
-    std::vector<uint64_t> words(e->W);
+    std::vector<uint64_t> v(e->nlimbs + 1);
     cudaSetDevice(e->device);
-    if (!kok(e, cudaMemcpyAsync(words.data(), x, (size_t)e->W * 8, cudaMemcpyDeviceToHost, e->stream)) ||
-        !kok(e, cudaStreamSynchronize(e->stream)))
-        return -1;
-    int st = 0;
-    if (!kok(e, cudaMemcpy(&st, e->d_status, sizeof st, cudaMemcpyDeviceToHost))) return -1;
-    if (st) {
-        e->err = -100 - st;
+    {
+        std::lock_guard<std::mutex> lock(e->out_mu);
+        uint64_t *out = e->d_out + e->W;
+        const int grid = (int)((e->nlimbs + 1 + 255) / 256);
+        launch(false, kn_reduce<true>, 1, kReduceThreads, 0, e->stream, e->d_desc, e->d_test, e->d_out, nullptr, x);
+        launch(true, kn_limbs, grid, 256, 0, e->stream, e->d_out, e->W, e->w, out, (uint32_t)e->nlimbs, e->d_status);
+        if (!kok(e, cudaGetLastError()) ||
+            !kok(e, cudaMemcpyAsync(v.data(), out, v.size() * 8, cudaMemcpyDeviceToHost, e->stream)) ||
+            !kok(e, cudaStreamSynchronize(e->stream)))
+            return -1;
+    }
+    if (v.back()) {
+        e->err = -100 - (int)v.back();
         return -1;
     }
-    from_mont(e, words.data(), limbs);
+    v.pop_back();
+    if (geq(v, e->N)) {
+        std::vector<uint64_t> r;
+        reduce_mod(e, v, r);
+        v.swap(r);
+    }
+    std::copy(v.begin(), v.end(), limbs);
     return 0;
 }
 
-static int run_product(kn_engine *e, uint64_t *x, const uint64_t *y, const uint64_t *addend) {
+// x <- x^2 (+ addend), `count` times, or x <- x y.  Between squarings the reduction is the next one's
+// column pass (Fold) where the number allows it.
+static int run_product(kn_engine *e, uint64_t *x, const uint64_t *y, const uint64_t *addend, uint64_t count) {
     const uint32_t R = e->plan->R, C = e->plan->C;
     const size_t col_smem = col_smem_bytes(R), row_smem = row_smem_bytes(C);
     const int ncols = (int)(C / kG), nrows = (int)R;
-    kn_col_fwd<<<ncols, kColThreads, col_smem, e->stream>>>(e->d_desc, e->d_cols, ncols, 0, x);
-    if (y) {
-        kn_col_fwd<<<ncols, kColThreads, col_smem, e->stream>>>(e->d_desc, e->d_cols, ncols, 1, y);
-        kn_rows<true><<<nrows, kRowThreads, 2 * row_smem, e->stream>>>(e->d_desc, e->d_rows, nrows);
-    } else {
-        kn_rows<false><<<nrows, kRowThreads, row_smem, e->stream>>>(e->d_desc, e->d_rows, nrows);
+    const int row_threads = std::max(64, std::min(kRowThreads, (int)e->np << ((ilog2(C) + 1) / 2)));
+    const uint64_t *none = nullptr;
+    for (uint64_t i = 0; i < count; i++) {
+        if (i && e->lazy) launch(true, kn_col_fwd<true>, ncols, kColThreads, col_smem, e->stream, e->d_desc, e->d_cols, ncols, 0, addend);
+        else launch(i > 0, kn_col_fwd<false>, ncols, kColThreads, col_smem, e->stream, e->d_desc, e->d_cols, ncols, 0, x);
+        if (y) {
+            launch(true, kn_col_fwd<false>, ncols, kColThreads, col_smem, e->stream, e->d_desc, e->d_cols, ncols, 1, y);
+            launch(true, kn_rows<true>, nrows, kRowThreads, 2 * row_smem, e->stream, e->d_desc, e->d_rows, nrows);
+        } else {
+            launch(true, kn_rows<false>, nrows, row_threads, row_smem, e->stream, e->d_desc, e->d_rows, nrows);
+        }
+        launch(true, kn_col_inv, ncols, kColThreads, col_smem, e->stream, e->d_desc, e->d_cols, ncols);
+        if (!e->lazy || i + 1 == count)
+            launch(true, kn_reduce<false>, 1, kReduceThreads, 0, e->stream, e->d_desc, e->d_test, x, addend, none);
+        if (!kok(e, cudaGetLastError())) return -1;
     }
-    kn_col_inv<<<ncols, kColThreads, col_smem, e->stream>>>(e->d_desc, e->d_cols, ncols);
-    kn_reduce<<<1, kReduceThreads, 0, e->stream>>>(e->d_desc, e->d_test, x, addend);
-    return kok(e, cudaGetLastError()) ? 0 : -1;
+    return 0;
 }
 
 int kn_square(kn_engine *e, uint64_t *x, uint64_t count) {
     if (!e || e->err) return -1;
     cudaSetDevice(e->device);
-    for (uint64_t i = 0; i < count; i++)
-        if (run_product(e, x, nullptr, nullptr)) return -1;
-    return 0;
+    return run_product(e, x, nullptr, nullptr, count);
 }
 
 int kn_square_add(kn_engine *e, uint64_t *x, uint64_t count, int64_t c) {
@@ -1214,15 +1451,13 @@ int kn_square_add(kn_engine *e, uint64_t *x, uint64_t count, int64_t c) {
         e->addend_c = c;
         e->addend_ok = true;
     }
-    for (uint64_t i = 0; i < count; i++)
-        if (run_product(e, x, nullptr, e->d_addend)) return -1;
-    return 0;
+    return run_product(e, x, nullptr, e->d_addend, count);
 }
 
 int kn_mul(kn_engine *e, uint64_t *x, const uint64_t *y) {
     if (!e || e->err) return -1;
     cudaSetDevice(e->device);
-    return run_product(e, x, y, nullptr);
+    return run_product(e, x, y, nullptr, 1);
 }
 
 int kn_copy(kn_engine *e, uint64_t *dst, const uint64_t *src) {
@@ -1258,6 +1493,7 @@ struct kn_group {
     size_t col_smem = 0, row_smem = 0;
     int grid = 0;
     int threads = 128;  // block size of the transform kernels
+    bool lazy = false;  // every member's numbers allow the reduction inside the column pass
     bool dirty = true;
     cudaGraphExec_t graph = nullptr;
     uint32_t graph_len = 0;
@@ -1295,11 +1531,13 @@ bool group_build(kn_group *g) {
     std::vector<int2> cols, rows;
     std::vector<int> tests(m);
     g->col_smem = g->row_smem = 0;
+    g->lazy = true;
     for (int t = 0; t < m; t++) {
         kn_engine *e = g->eng[order[t]];
         descs[t] = e->desc;
         descs[t].x = g->xs[order[t]];
         descs[t].addend = nullptr;
+        g->lazy = g->lazy && e->lazy;
         tests[t] = t;
         for (uint32_t c = 0; c < e->plan->C / kG; c++) cols.push_back(make_int2(t, (int)c));
         for (uint32_t r = 0; r < e->plan->R; r++) rows.push_back(make_int2(t, (int)r));
@@ -1325,13 +1563,19 @@ bool group_build(kn_group *g) {
     return ok;
 }
 
-void group_square_once(kn_group *g) {
-    const int gc = std::min(g->ncols, g->grid), gr = std::min(g->nrows, g->grid);
-    kn_col_fwd<<<gc, g->threads, g->col_smem, g->stream>>>(g->d_desc, g->d_cols, g->ncols, 0, nullptr);
-    // a row item is 4 B units per register pass (B = 16 for the common C = 256): 64 threads
-    kn_rows<false><<<std::min(g->nrows, 2 * g->grid), 64, g->row_smem, g->stream>>>(g->d_desc, g->d_rows, g->nrows);
-    kn_col_inv<<<gc, g->threads, g->col_smem, g->stream>>>(g->d_desc, g->d_cols, g->ncols);
-    kn_reduce<<<g->ntests, kReduceThreads, 0, g->stream>>>(g->d_desc, g->d_tests, nullptr, nullptr);
+// `count` squarings of every member.  The reduction is the next squaring's column pass (Fold) where
+// every member allows it, and a pass of its own after the last one.
+void group_square_run(kn_group *g, uint64_t count) {
+    const int gc = std::min(g->ncols, g->grid);
+    for (uint64_t i = 0; i < count; i++) {
+        launch(i > 0, i && g->lazy ? kn_col_fwd<true> : kn_col_fwd<false>, gc, g->threads, g->col_smem, g->stream, g->d_desc,
+               g->d_cols, g->ncols, 0, nullptr);
+        // a row item is 4 B units per register pass (B = 16 for the common C = 256): 64 threads
+        launch(true, kn_rows<false>, std::min(g->nrows, 2 * g->grid), 64, g->row_smem, g->stream, g->d_desc, g->d_rows, g->nrows);
+        launch(true, kn_col_inv, gc, g->threads, g->col_smem, g->stream, g->d_desc, g->d_cols, g->ncols);
+        if (!g->lazy || i + 1 == count)
+            launch(true, kn_reduce<false>, g->ntests, kReduceThreads, 0, g->stream, g->d_desc, g->d_tests, nullptr, nullptr, nullptr);
+    }
 }
 
 constexpr uint32_t kGroupChunk = 8;  // squarings per captured graph
@@ -1388,7 +1632,7 @@ bool group_prepare(kn_group *g) {
     if (!g->graph) {
         cudaGraph_t graph = nullptr;
         if (!gok(g, cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal))) return false;
-        for (uint32_t i = 0; i < kGroupChunk; i++) group_square_once(g);
+        group_square_run(g, kGroupChunk);
         if (!gok(g, cudaStreamEndCapture(g->stream, &graph))) return false;
         const bool ok = gok(g, cudaGraphInstantiate(&g->graph, graph, 0));
         cudaGraphDestroy(graph);
@@ -1431,8 +1675,8 @@ int kn_groups_square(kn_group *const *gs, int ng, uint64_t count, float *gpu_ms)
     uint64_t done = 0;
     for (; ok && done + kGroupChunk <= count; done += kGroupChunk)
         for (kn_group *g : live) ok = ok && gok(g, cudaGraphLaunch(g->graph, g->stream));
-    for (; ok && done < count; done++)
-        for (kn_group *g : live) group_square_once(g);
+    for (kn_group *g : live)
+        if (ok) group_square_run(g, count - done);
     for (kn_group *g : live)
         if (ok && g != g0)
             ok = gok(g, cudaEventRecord(g->ev1, g->stream)) && gok(g0, cudaStreamWaitEvent(g0->stream, g->ev1, 0));
@@ -1458,7 +1702,7 @@ int kn_group_square(kn_group *g, uint64_t count, float *gpu_ms) {
     uint64_t done = 0;
     for (; done + g->graph_len <= count; done += g->graph_len)
         if (!gok(g, cudaGraphLaunch(g->graph, g->stream))) return -1;
-    for (; done < count; done++) group_square_once(g);
+    group_square_run(g, count - done);
     gok(g, cudaEventRecord(g->ev1, g->stream));
     if (!gok(g, cudaGetLastError()) || !gok(g, cudaStreamSynchronize(g->stream))) return -1;
     if (gpu_ms) cudaEventElapsedTime(gpu_ms, g->ev0, g->ev1);
@@ -1477,11 +1721,11 @@ int kn_group_mul(kn_group *g, const uint64_t *const *ys, float *gpu_ms) {
         return -1;
     const int gc = std::min(g->ncols, g->grid), gr = std::min(g->nrows, 2 * g->grid);
     gok(g, cudaEventRecord(g->ev0, g->stream));
-    kn_col_fwd<<<gc, g->threads, g->col_smem, g->stream>>>(g->d_desc, g->d_cols, g->ncols, 0, nullptr);
-    kn_col_fwd<<<gc, g->threads, g->col_smem, g->stream>>>(g->d_desc, g->d_cols, g->ncols, 1, nullptr);
+    kn_col_fwd<false><<<gc, g->threads, g->col_smem, g->stream>>>(g->d_desc, g->d_cols, g->ncols, 0, nullptr);
+    kn_col_fwd<false><<<gc, g->threads, g->col_smem, g->stream>>>(g->d_desc, g->d_cols, g->ncols, 1, nullptr);
     kn_rows<true><<<gr, 64, 2 * g->row_smem, g->stream>>>(g->d_desc, g->d_rows, g->nrows);
     kn_col_inv<<<gc, g->threads, g->col_smem, g->stream>>>(g->d_desc, g->d_cols, g->ncols);
-    kn_reduce<<<g->ntests, kReduceThreads, 0, g->stream>>>(g->d_desc, g->d_tests, nullptr, nullptr);
+    kn_reduce<false><<<g->ntests, kReduceThreads, 0, g->stream>>>(g->d_desc, g->d_tests, nullptr, nullptr, nullptr);
     gok(g, cudaEventRecord(g->ev1, g->stream));
     if (!gok(g, cudaGetLastError()) || !gok(g, cudaStreamSynchronize(g->stream))) return -1;
     if (gpu_ms) cudaEventElapsedTime(gpu_ms, g->ev0, g->ev1);
