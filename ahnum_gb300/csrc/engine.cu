@@ -92,6 +92,7 @@ void release(kc_engine *e) {
     cudaFree(e->d_slot);
     cudaFree(e->d_maxerr);
     cudaFree(e->d_rexp);
+    cudaFree(e->d_flags);
     if (e->h_dig) cudaFreeHost(e->h_dig);
     if (e->h_err) cudaFreeHost(e->h_err);
     if (e->stream) cudaStreamDestroy(e->stream);
@@ -138,8 +139,9 @@ int product(kc_engine *e, double2 *x, const double2 *y) {
     return check_launch(e) ? 0 : e->err;
 }
 
-// Chains wait on their own CTAs, so two of them must not be on the device at once: each one is put
-// behind the previous one of the device, whichever engine launched it.
+// Cooperative chains wait on their own CTAs, so two of them must not be on the device at once: each one
+// is put behind the previous one of the device, whichever engine launched it.  A cluster's CTAs start
+// together and need none of this.
 struct ChainQueue {
     std::mutex mu;
     cudaEvent_t last = nullptr;
@@ -152,14 +154,23 @@ int square_many(kc_engine *e, double2 *x, uint64_t count) {
     ChainQueue &q = g_chains[e->device];
     while (count) {
         const int n = (int)std::min(count, kChainSteps);
+        if (e->chain_cluster) {
+            if (!ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, true, x, (int)(e->op_count % e->err_every), n, e->d_chain, 0, nullptr, 0)))
+                return e->err;
+            e->op_count += (uint64_t)n;
+            count -= (uint64_t)n;
+            continue;
+        }
         std::lock_guard<std::mutex> lock(q.mu);
         if (!q.last && !ok(e, cudaEventCreateWithFlags(&q.last, cudaEventDisableTiming))) return e->err;
         if (q.stream != e->stream && !ok(e, cudaStreamWaitEvent(e->stream, q.last, 0))) return e->err;
-        if (!ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, x, (int)(e->op_count % e->err_every), n, e->d_chain, e->arrived)) ||
+        if (!ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, false, x, (int)(e->op_count % e->err_every), n, e->d_chain, e->arrived,
+                                e->d_flags, e->chained)) ||
             !ok(e, cudaEventRecord(q.last, e->stream)))
             return e->err;
         q.stream = e->stream;
-        e->arrived += 3u * (unsigned)n * (unsigned)e->chain_grid;
+        e->arrived += 2u * (unsigned)n * (unsigned)e->chain_grid;
+        e->chained += (unsigned)n;
         e->op_count += (uint64_t)n;
         count -= (uint64_t)n;
     }
@@ -253,14 +264,14 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
     const LengthPlan &P = *e->plan;
     const uint32_t H = P.H;
     e->NG = P.C / e->G;
-    const size_t chain_at = ((size_t)P.R + 2) & ~(size_t)1;  // the chain's words after the exponents, aligned
+    const size_t chain_at = ((size_t)P.R + 3) & ~(size_t)1;  // the chain's words after the exponents and emax, aligned
     bool good = ok(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) &&
                 dalloc(e, &e->d_desc, 1) && dalloc(e, &e->d_work, P.pairs.size() + e->NG) &&
                 dalloc(e, &e->d_bits, L) && dalloc(e, &e->d_w, L) && dalloc(e, &e->d_osc, L) &&
                 dalloc(e, &e->d_idig, L) && dalloc(e, &e->d_dig, L) && dalloc(e, &e->d_dig2, L) &&
                 dalloc(e, &e->d_eq, 1) && ok(e, cudaMallocHost((void **)&e->h_eq, sizeof(int))) &&
                 dalloc(e, &e->d_slot, (size_t)e->NG * P.R) &&
-                dalloc(e, &e->d_maxerr, 1) && dalloc(e, &e->d_rexp, chain_at + sizeof(ChainCtl) / sizeof(int)) &&
+                dalloc(e, &e->d_maxerr, 1) && dalloc(e, &e->d_flags, (size_t)e->NG * kFlagWords) && dalloc(e, &e->d_rexp, chain_at + sizeof(ChainCtl) / sizeof(int)) &&
                 ok(e, cudaMallocHost((void **)&e->h_dig, (size_t)L * sizeof(long long))) &&
                 ok(e, cudaMallocHost((void **)&e->h_err, 2 * sizeof(unsigned long long)));
     if (good) {
@@ -274,7 +285,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
             osc[j] = fixed_ratio(ms, wv[j], inv);
             idig[j] = fixed_ratio(mi, wv[j], inv);
         }
-        const int emax0 = INT_MIN;
+        const int emax0[2] = {INT_MIN, INT_MIN};
         e->h_timeout = reinterpret_cast<unsigned *>(e->h_err + 1);
         *e->h_timeout = 0;
         e->d_chain = reinterpret_cast<ChainCtl *>(e->d_rexp + chain_at);
@@ -288,7 +299,8 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
                ok(e, cudaMemcpy(e->d_idig, idig.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemcpy(e->d_work, work.data(), work.size() * sizeof(WorkItem), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemset(e->d_maxerr, 0, sizeof(unsigned long long))) &&
-               ok(e, cudaMemcpy(e->d_rexp + P.R, &emax0, sizeof(int), cudaMemcpyHostToDevice)) &&
+               ok(e, cudaMemcpy(e->d_rexp + P.R, emax0, sizeof emax0, cudaMemcpyHostToDevice)) &&
+               ok(e, cudaMemset(e->d_flags, 0, (size_t)e->NG * kFlagWords * sizeof(unsigned))) &&
                ok(e, cudaMemcpy(e->d_chain, &chain0, sizeof chain0, cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemset(e->d_slot, 0, (size_t)e->NG * P.R * sizeof(long long)));
     }
@@ -342,10 +354,11 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         s.row_smem_per_lane = (size_t)P.C * sizeof(longlong2);
         s.col_smem = 2 * (size_t)P.R * e->G * sizeof(longlong2);
         s.G = e->G;
-        // twiddles of both plans, split twiddles of a row; t4, osc, w of a column group, its widths
-        s.table_smem = ((size_t)2 * P.C + P.R + 3 * (size_t)P.R * e->G) * 16 + ((size_t)2 * P.R * e->G + 15) / 16 * 16;
+        // twiddles of both plans, split twiddles of a row; t4, osc, w, digits of a column group, its widths
+        s.table_smem = ((size_t)2 * P.C + P.R + 4 * (size_t)P.R * e->G) * 16 + ((size_t)2 * P.R * e->G + 15) / 16 * 16;
         good = good && ok(e, cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device)) &&
                kernels_prepare(s.row_smem_per_lane * 6, s.col_smem, chain_smem(s, e->nsm)) == 0;
+        e->chain_cluster = chain_in_cluster(s);
         e->chain_grid = good ? chain_grid(s, e->nsm) : 0;
         good = e->chain_grid > 0;
     }
@@ -546,7 +559,7 @@ int kc_engine_wait_selftest(kc_engine *e, uint64_t wait_cycles) {
     rc = -1;
     if (x && ok(e, cudaMalloc((void **)&ctl, sizeof(ChainCtl))) &&
         ok(e, cudaMemcpyAsync(ctl, &c0, sizeof c0, cudaMemcpyHostToDevice, e->stream)) &&
-        ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, (double2 *)x, 0, 1, ctl, 1, (long long)wait_cycles)) &&
+        ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, false, (double2 *)x, 0, 1, ctl, 1, e->d_flags, e->chained, (long long)wait_cycles)) &&
         ok(e, cudaMemcpyAsync(&c1, ctl, sizeof c1, cudaMemcpyDeviceToHost, e->stream)) &&
         ok(e, cudaMemcpyAsync(e->d_rexp + e->plan->R, &emax0, sizeof emax0, cudaMemcpyHostToDevice, e->stream)) &&
         ok(e, cudaStreamSynchronize(e->stream)))

@@ -39,6 +39,9 @@ struct kc_engine {
     kg::ChainCtl *d_chain = nullptr;   // squaring chains: device words
     unsigned *h_timeout = nullptr;     //   pinned, after h_err: non-zero once a wait in one gave up
     unsigned arrived = 0;              //   arrivals at the barrier so far
+    unsigned *d_flags = nullptr;       //   of each column group, at `chained`, the squarings so far
+    unsigned chained = 0;
+    bool chain_cluster = false;
     int chain_grid = 0, nsm = 0;
 };
 

@@ -210,16 +210,25 @@ __device__ __forceinline__ longlong2 quarter(longlong2 a, long long half) {
 }
 
 // How a pass reads the tables: in global memory (the read-only path), or wherever they are (the chain
-// keeps its own slices in shared memory).
+// keeps its own slices in shared memory); and the digits that the first half of a column pass left for
+// the second one, which another CTA may have written unless the chain says otherwise.
 struct GlobalTables {
     template <class V>
     static __device__ __forceinline__ V load(const V *p) {
         return __ldg(p);
     }
+    template <class V>
+    static __device__ __forceinline__ V load_own(const V *p) {
+        return __ldcg(p);
+    }
 };
 struct AnyTables {
     template <class V>
     static __device__ __forceinline__ V load(const V *p) {
+        return *p;
+    }
+    template <class V>
+    static __device__ __forceinline__ V load_own(const V *p) {
         return *p;
     }
 };

@@ -92,11 +92,16 @@ struct ChainCtl {
     unsigned *host_timeout;
 };
 // `nsteps` squarings of x (squaring step0, step0 + 1, ... for the tracking of round-off) in one
-// cooperative launch of `grid` CTAs (chain_grid), which arrive 3 nsteps times each at ctl->arrived,
-// `arrived` before the launch.
-cudaError_t launch_chain(const LaunchSet &s, int nsm, int grid, double2 *x, int step0, int nsteps, ChainCtl *ctl, unsigned arrived,
-                         long long limit = kWaitCycles);
-// CTAs of a chain: one per item of the larger pass, at most what is resident at once; 0 on failure.
+// launch of `grid` CTAs (chain_grid), as one cluster or cooperatively.  In the second case they arrive
+// 2 nsteps times each at ctl->arrived, `arrived` before the launch, and raise each column group's flag
+// (kFlagWords apart) from `done` to done + nsteps.
+constexpr int kFlagWords = 8;      // one 32-byte sector
+constexpr int kClusterItems = 16;  // the largest cluster
+cudaError_t launch_chain(const LaunchSet &s, int nsm, int grid, bool cluster, double2 *x, int step0, int nsteps, ChainCtl *ctl,
+                         unsigned arrived, unsigned *flags, unsigned done, long long limit = kWaitCycles);
+bool chain_in_cluster(const LaunchSet &s);
+// CTAs of a chain: one per item of the larger pass (a power of two in a cluster), at most what is
+// resident at once; 0 on failure.
 int chain_grid(const LaunchSet &s, int nsm);
 size_t chain_smem(const LaunchSet &s, int nsm);  // its dynamic shared memory
 int chain_set_smem(size_t bytes);

@@ -501,7 +501,7 @@ __device__ __forceinline__ void segment_carries(const TestDesc &T, int g, const 
         }
         const bool top = g == T.NG - 1 && r == R - 1;
         if (top) cy = fold_segment<G>(T, bw, d, cy);
-        longlong2 *dst = reinterpret_cast<longlong2 *>(T.dig + j0);  // j0 is even
+        longlong2 *dst = reinterpret_cast<longlong2 *>(T.dig + 2 * (r * T.pitch + g * G));
 #pragma unroll
         for (int l = 0; l < G; l++) dst[l] = make_longlong2(d[2 * l], d[2 * l + 1]);
         T.slot[top ? 0 : g < T.NG - 1 ? (g + 1) * R + r : r + 1] = cy;
@@ -558,16 +558,15 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
 
 template <int G, class TAB>
 __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool use_slots, int shift, longlong2 *sm) {
-    const int R = T.R, C = T.C;
+    const int R = T.R;
     constexpr int LG = G == 8 ? 3 : G == 4 ? 2 : 1;
     // absorb the carry-in into the segment's first digits (the last digit takes any rest), reweight
     for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        const int j0 = 2 * (r * C + g * G);
         long long d[2 * G];
-        const longlong2 *src = reinterpret_cast<const longlong2 *>(T.dig + j0);  // j0 is even
+        const longlong2 *src = reinterpret_cast<const longlong2 *>(T.dig + 2 * (r * T.pitch + g * G));
 #pragma unroll
         for (int l = 0; l < G; l++) {
-            const longlong2 p = __ldcg(src + l);
+            const longlong2 p = TAB::load_own(src + l);
             d[2 * l] = p.x;
             d[2 * l + 1] = p.y;
         }

@@ -114,29 +114,36 @@ static double stage_rounds(uint32_t n, uint32_t count) {
     return sum;
 }
 
-// Predicted time in us of one squaring of a chain (chain.cu) of R x C in column groups of G, from
-// what every CTA does in a row: fitted to 310 shapes of 21 lengths from 512 to 1769472 digits.
-//  - a fixed part, mostly the three grid barriers and the first loads after them;
-//  - the rounds of a row pair's and a column group's stages, there and back, and the rounds over their
-//    points besides (loads, squares, carries; a column group has two such passes);
+// Predicted time in us of one squaring of a chain (chain.cuh) of R x C in column groups of G, from
+// what every CTA does in a row: fitted to 420 shapes of 23 lengths from 320 to 1769472 digits, whose
+// choices are within 1.6% of the best shape on average.
+// In one cluster: the rounds of a row pair's and a column group's stages, there and back, and the digits
+// of a segment, whose carries are serial.  Up to 2048 digits only: from 3072 on a cluster's wide groups
+// lose to narrow ones on more CTAs (13.6 against 12.6 us).  On the whole GPU:
+//  - a fixed part, mostly the two grid barriers, the wait for a neighbour and the loads after them;
+//  - the same rounds, and the rounds over the items' points besides (loads, squares, carries; a column
+//    group has two such passes);
 //  - 1.6 times that in a wave which puts two CTAs on an SM: alone, a CTA waits for its own latencies;
 //  - a wave more wherever a pass has more items than CTAs stay: one per SM, or two up to kTwoCtaSmem;
 //  - the tables read from L2 when they do not stay in shared memory.
 static double chain_us(uint32_t R, uint32_t C, int G, int nsm) {
     constexpr size_t kTwoCtaSmem = 108 * 1024;
+    constexpr double kFixed = 6.18, kRound = 0.435, kPoints = 0.547, kWave = 3.14, kFromL2 = 4.8, kPerLog = 0.23;
     const uint32_t pairs = R / 2 + 1, groups = C / G, most = std::max(pairs, groups);
+    if (most <= (uint32_t)kClusterItems)
+        return 3.17 + 0.684 * 2 * (stage_rounds(C, 2) + stage_rounds(R, G)) + 0.444 * G + (R * C > 1024 ? 1e2 : 0);
     const size_t smem = 16 * std::max((size_t)4 * C, (size_t)2 * R * G);
-    const size_t table = 16 * ((size_t)2 * C + R + (size_t)3 * R * G) + (size_t)2 * R * G;
+    const size_t table = 16 * ((size_t)2 * C + R + (size_t)4 * R * G) + (size_t)2 * R * G;
     const bool keeps = most <= (uint32_t)nsm && smem + table <= kMaxChainSmem;
     const uint32_t resident = std::min<uint32_t>(most, nsm * (!keeps && smem <= kTwoCtaSmem ? 2 : 1));
     const auto pass = [&](uint32_t items, uint32_t n, uint32_t count, double passes) {
-        double us = -2.16 * passes;
-        const double once = 0.475 * 2 * stage_rounds(n, count) + 0.54 * passes * ((count * n + kThreads - 1) / kThreads);
+        double us = -kWave * passes;
+        const double once = kRound * 2 * stage_rounds(n, count) + kPoints * passes * ((count * n + kThreads - 1) / kThreads);
         for (uint32_t left = items; left; left -= std::min(left, resident))
-            us += 2.16 * passes + once * (std::min(left, resident) > (uint32_t)nsm ? 1.6 : 1.0);
+            us += kWave * passes + once * (std::min(left, resident) > (uint32_t)nsm ? 1.6 : 1.0);
         return us;
     };
-    return 6.75 + pass(pairs, C, 2, 1) + pass(groups, R, G, 2) + (keeps ? 0 : 3.1) + 0.18 * std::log2((double)R);
+    return kFixed + pass(pairs, C, 2, 1) + pass(groups, R, G, 2) + (keeps ? 0 : kFromL2) + kPerLog * std::log2((double)R);
 }
 
 // Latency shapes chosen by the autotuner (or a tuning file), by FFT length L = 2H: (R, G).
