@@ -33,6 +33,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <tuple>
 #include <vector>
 
 #include "../../include/kite_ntt.h"
@@ -882,19 +883,28 @@ void level_table(std::vector<uint2> &out, uint32_t n, uint32_t wn, uint32_t p) {
 }
 
 std::mutex g_plan_mu;
-std::map<std::pair<int, uint32_t>, std::shared_ptr<Plan>> g_plans;
+std::map<std::tuple<int, uint32_t, uint32_t>, std::shared_ptr<Plan>> g_plans;
 
-std::shared_ptr<Plan> get_plan(int device, uint32_t NP) {
+// Rows of the R x C layout.  Many tests: as square as it gets, which is the least work per word.  One test
+// alone: half as many rows (at most 1024 columns, at least 8 rows), since a column pass has only C / 8
+// CTAs: on GB300, us per squaring alone at n = 20000, 369717, 1500000: 13.9, 20.6, 30.9 square and
+// 13.7, 16.9, 23.7 so (12.4, 17.9, 25.2 with a quarter of the rows); 128 tests on two streams 166 us
+// square and 181 us so.
+uint32_t plan_rows(uint32_t NP, bool alone) {
+    const uint32_t square = 1u << (ilog2(NP) / 2);
+    return alone && square > 8 && NP / square < 1024 ? square / 2 : square;
+}
+
+std::shared_ptr<Plan> get_plan(int device, uint32_t NP, uint32_t R) {
     std::lock_guard<std::mutex> lock(g_plan_mu);
-    auto key = std::make_pair(device, NP);
+    auto key = std::make_tuple(device, NP, R);
     auto itp = g_plans.find(key);
     if (itp != g_plans.end()) return itp->second;
     auto P = std::make_shared<Plan>();
     P->NP = NP;
-    const int a = ilog2(NP);
-    P->R = 1u << (a / 2);
-    P->C = NP / P->R;
-    const uint32_t R = P->R, C = P->C;
+    P->R = R;
+    P->C = NP / R;
+    const uint32_t C = P->C;
     const int logR = ilog2(R);
     // layout per prime: twr_f[R], twr_i[R], twc_f[C], twc_i[C], t4_f[NP], t4_i[NP]
     const size_t per = 2 * (size_t)R + 2 * (size_t)C + 2 * (size_t)NP;
@@ -1258,7 +1268,7 @@ kn_engine *kn_engine_new(uint64_t k, uint64_t n, int device) {
         delete e;
         return nullptr;
     }
-    e->plan = get_plan(device, e->NP);
+    e->plan = get_plan(device, e->NP, plan_rows(e->NP, true));
     if (!e->plan) {
         delete e;
         return nullptr;
@@ -1486,6 +1496,7 @@ struct kn_group {
     std::vector<uint64_t *> xs;
     std::vector<Desc> h_desc;  // the device table's host copy, in work-list order
     std::vector<int> slot;     // member -> its index in the table
+    std::vector<std::shared_ptr<Plan>> plans;  // of the descriptors, in the same order
     Desc *d_desc = nullptr;
     int2 *d_cols = nullptr, *d_rows = nullptr;
     int *d_tests = nullptr;
@@ -1532,17 +1543,24 @@ bool group_build(kn_group *g) {
     std::vector<int> tests(m);
     g->col_smem = g->row_smem = 0;
     g->lazy = true;
+    g->plans.clear();
     for (int t = 0; t < m; t++) {
         kn_engine *e = g->eng[order[t]];
         descs[t] = e->desc;
         descs[t].x = g->xs[order[t]];
+        const std::shared_ptr<Plan> plan = get_plan(g->device, e->NP, plan_rows(e->NP, false));
+        if (!plan) return gok(g, cudaErrorMemoryAllocation);
+        g->plans.push_back(plan);
+        descs[t].R = plan->R;
+        descs[t].C = plan->C;
+        descs[t].tb = plan->tb;
         descs[t].addend = nullptr;
         g->lazy = g->lazy && e->lazy;
         tests[t] = t;
-        for (uint32_t c = 0; c < e->plan->C / kG; c++) cols.push_back(make_int2(t, (int)c));
-        for (uint32_t r = 0; r < e->plan->R; r++) rows.push_back(make_int2(t, (int)r));
-        g->col_smem = std::max(g->col_smem, col_smem_bytes(e->plan->R));
-        g->row_smem = std::max(g->row_smem, row_smem_bytes(e->plan->C));
+        for (uint32_t c = 0; c < plan->C / kG; c++) cols.push_back(make_int2(t, (int)c));
+        for (uint32_t r = 0; r < plan->R; r++) rows.push_back(make_int2(t, (int)r));
+        g->col_smem = std::max(g->col_smem, col_smem_bytes(plan->R));
+        g->row_smem = std::max(g->row_smem, row_smem_bytes(plan->C));
     }
     g->ncols = (int)cols.size();
     g->nrows = (int)rows.size();
