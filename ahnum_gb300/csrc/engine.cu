@@ -92,7 +92,6 @@ void release(kc_engine *e) {
     cudaFree(e->d_slot);
     cudaFree(e->d_maxerr);
     cudaFree(e->d_rexp);
-    cudaFree(e->d_flags);
     if (e->h_dig) cudaFreeHost(e->h_dig);
     if (e->h_err) cudaFreeHost(e->h_err);
     if (e->stream) cudaStreamDestroy(e->stream);
@@ -264,14 +263,15 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
     const LengthPlan &P = *e->plan;
     const uint32_t H = P.H;
     e->NG = P.C / e->G;
-    const size_t chain_at = ((size_t)P.R + 3) & ~(size_t)1;  // the chain's words after the exponents and emax, aligned
+    // the chain's words after the exponents and emax, aligned; its flags after those
+    const size_t chain_at = ((size_t)P.R + 3) & ~(size_t)1, flags_at = (chain_at + sizeof(ChainCtl) / sizeof(int) + 7) & ~(size_t)7;
     bool good = ok(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) &&
                 dalloc(e, &e->d_desc, 1) && dalloc(e, &e->d_work, P.pairs.size() + e->NG) &&
                 dalloc(e, &e->d_bits, L) && dalloc(e, &e->d_w, L) && dalloc(e, &e->d_osc, L) &&
                 dalloc(e, &e->d_idig, L) && dalloc(e, &e->d_dig, L) && dalloc(e, &e->d_dig2, L) &&
                 dalloc(e, &e->d_eq, 1) && ok(e, cudaMallocHost((void **)&e->h_eq, sizeof(int))) &&
                 dalloc(e, &e->d_slot, (size_t)e->NG * P.R) &&
-                dalloc(e, &e->d_maxerr, 1) && dalloc(e, &e->d_flags, (size_t)e->NG * kFlagWords) && dalloc(e, &e->d_rexp, chain_at + sizeof(ChainCtl) / sizeof(int)) &&
+                dalloc(e, &e->d_maxerr, 1) && dalloc(e, &e->d_rexp, flags_at + (size_t)e->NG * kFlagWords) &&
                 ok(e, cudaMallocHost((void **)&e->h_dig, (size_t)L * sizeof(long long))) &&
                 ok(e, cudaMallocHost((void **)&e->h_err, 2 * sizeof(unsigned long long)));
     if (good) {
@@ -285,11 +285,14 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
             osc[j] = fixed_ratio(ms, wv[j], inv);
             idig[j] = fixed_ratio(mi, wv[j], inv);
         }
-        const int emax0[2] = {INT_MIN, INT_MIN};
         e->h_timeout = reinterpret_cast<unsigned *>(e->h_err + 1);
         *e->h_timeout = 0;
         e->d_chain = reinterpret_cast<ChainCtl *>(e->d_rexp + chain_at);
+        e->d_flags = reinterpret_cast<unsigned *>(e->d_rexp + flags_at);
+        std::vector<int> words(flags_at + (size_t)e->NG * kFlagWords - P.R, 0);  // from emax on
+        words[0] = words[1] = INT_MIN;
         const ChainCtl chain0{0, 0, e->h_timeout};
+        std::memcpy(words.data() + chain_at - P.R, &chain0, sizeof chain0);
         std::vector<WorkItem> work;
         for (size_t i = 0; i < P.pairs.size(); i++) work.push_back({0, (int)i});
         for (uint32_t g = 0; g < e->NG; g++) work.push_back({0, (int)g});
@@ -299,9 +302,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
                ok(e, cudaMemcpy(e->d_idig, idig.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemcpy(e->d_work, work.data(), work.size() * sizeof(WorkItem), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemset(e->d_maxerr, 0, sizeof(unsigned long long))) &&
-               ok(e, cudaMemcpy(e->d_rexp + P.R, emax0, sizeof emax0, cudaMemcpyHostToDevice)) &&
-               ok(e, cudaMemset(e->d_flags, 0, (size_t)e->NG * kFlagWords * sizeof(unsigned))) &&
-               ok(e, cudaMemcpy(e->d_chain, &chain0, sizeof chain0, cudaMemcpyHostToDevice)) &&
+               ok(e, cudaMemcpy(e->d_rexp + P.R, words.data(), words.size() * sizeof(int), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemset(e->d_slot, 0, (size_t)e->NG * P.R * sizeof(long long)));
     }
     if (good) {

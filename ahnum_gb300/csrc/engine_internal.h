@@ -26,7 +26,7 @@ struct kc_engine {
     long long *d_dig2 = nullptr;     // second digit vector of the zero test (kc_equal)
     int *d_eq = nullptr, *h_eq = nullptr;  // its verdict, on the device and pinned
     unsigned long long *d_maxerr = nullptr;
-    int *d_rexp = nullptr;           // R row exponents, the test's largest (TestDesc::emax), *d_chain
+    int *d_rexp = nullptr;           // R row exponents, the test's largest (TestDesc::emax, two words), *d_chain, d_flags
     long long *h_dig = nullptr;      // pinned staging for digit transfers
     unsigned long long *h_err = nullptr;
     int err = 0;
