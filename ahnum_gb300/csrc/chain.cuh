@@ -78,6 +78,7 @@ __device__ __forceinline__ void keep(void *dst, const void *src, int count) {
 template <int LG>
 __device__ __forceinline__ void keep_tables(TestDesc *d, longlong2 *buf, int unit, int at) {
     const int R = d->R, C = d->C, G = 1 << LG, points = R << LG;
+    const ptrdiff_t first = (ptrdiff_t)unit << LG;  // the group's first column
     int4 *twr = reinterpret_cast<int4 *>(buf + at), *twc = twr + C, *sw = twc + R, *t4 = sw + C;
     int4 *osc = t4 + points, *w = osc + points, *dig = w + points, *bits = dig + points;
     keep(twr, d->twr, C - 1);
@@ -89,22 +90,22 @@ __device__ __forceinline__ void keep_tables(TestDesc *d, longlong2 *buf, int uni
             const size_t e = (size_t)(i >> LG) * C + (unit << LG) + (i & (G - 1));
             t4[i] = __ldg(d->t4 + e);
             osc[i] = __ldg(reinterpret_cast<const int4 *>(d->osc) + e);
-            w[i] = __ldg(reinterpret_cast<const int4 *>(d->w) + e);
-            reinterpret_cast<unsigned short *>(bits)[i] = __ldg(reinterpret_cast<const unsigned short *>(d->bits) + e);
         }
+        keep(w, reinterpret_cast<const int4 *>(d->w) + first * R, points);
+        const unsigned *widths = reinterpret_cast<const unsigned *>(d->segbits + 2 * first * R);
+        for (int i = threadIdx.x; i < points / 2; i += blockDim.x) reinterpret_cast<unsigned *>(bits)[i] = __ldg(widths + i);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const ptrdiff_t first = (ptrdiff_t)unit << LG;  // the group's first column
         d->twr = twr;
         d->twc = twc;
         d->sw = sw - (ptrdiff_t)row * C;
         d->pitch = G;
         d->t4 = t4 - first;
         d->osc = reinterpret_cast<long long *>(osc - first);
-        d->w = reinterpret_cast<long long *>(w - first);
-        d->bits = reinterpret_cast<uint8_t *>(bits) - 2 * first;
-        d->dig = reinterpret_cast<long long *>(dig - first);
+        d->w = reinterpret_cast<long long *>(w - first * R);
+        d->segbits = reinterpret_cast<uint8_t *>(bits) - 2 * first * R;
+        d->dig = reinterpret_cast<long long *>(dig - first * R);
     }
     __syncthreads();
 }

@@ -17,7 +17,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_col_forward(const Test
     if (nwork_dev) nwork = *nwork_dev;
     walk_items(
         tests, work, nwork, step, &s_desc, &s_ctl,
-        [](const TestDesc &T, int g) { touch_columns(T, g, T.w); },
         [&](const TestDesc &T, int g) {
             col_forward_item<LG, GlobalTables>(T, g, xo ? xo : T.x, use_slots != 0, digit_bits > 0 ? digit_bits : T.digit_bits, sm, s_ctl);
         });

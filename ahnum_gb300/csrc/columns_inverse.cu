@@ -18,7 +18,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_col_inverse(const Test
     if (nwork_dev) nwork = *nwork_dev;
     walk_items(
         tests, work, nwork, step, &s_desc, &s_ctl,
-        [](const TestDesc &T, int g) { touch_columns(T, g, T.osc); },
         [&](const TestDesc &T, int g) { col_inverse_item<LG, GlobalTables>(T, g, step, xo ? xo : T.x, sm, s_ctl); });
 }
 
@@ -31,7 +30,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_col_digits(const TestD
     __shared__ ItemCtl s_ctl;
     walk_items(
         tests, work, nwork, 0, &s_desc, &s_ctl,
-        [](const TestDesc &T, int g) { touch_columns(T, g, T.idig); },
         [&](const TestDesc &T, int g) { col_digits_item<LG, GlobalTables>(T, g, xo ? xo : T.x, digo ? digo : T.dig, sm, s_ctl); });
 }
 

@@ -58,14 +58,16 @@ struct alignas(16) TestDesc {
     int npairs;
     // per-modulus tables, 64-bit fixed point
     const uint8_t *bits;     // [L]
-    const long long *w;      // [L] weights w_j 2^61
+    const uint8_t *segbits;  // [g][row][2G] the same, by column group: the widths of a row segment
+    const long long *w;      // [column][row][2] weights w_j 2^61
     const long long *osc;    // [L] k / (w_j * 4H) 2^(62 - osc_exp): unweight and scale after a product
     const long long *idig;   // [L] 1 / (R * w_j) 2^(62 - idig_exp): unweight after the column inverse alone
     int osc_exp, idig_exp;
-    int pitch;               // columns from one row to the next of t4, osc, w and bits: C
+    int pitch;               // columns from one row to the next of t4 and osc: C
     int digit_bits;          // digits entering the column forward pass stay below 2^digit_bits
     // scratch
-    long long *dig;          // [L] integer digits between the two column kernels
+    long long *dig;          // [L] integer digits: a number's in their order, or between the two column
+                             // kernels [column][row][2]
     long long *slot;         // [NG * R] carry into segment (g, r), index g*R + r
     unsigned long long *maxerr;  // bits of the largest round-off (non-negative double)
     int *rexp;               // [R] the row pass leaves row k_r as fixed-point numbers times 2^rexp[k_r]

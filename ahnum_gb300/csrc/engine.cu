@@ -267,7 +267,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
     const size_t chain_at = ((size_t)P.R + 3) & ~(size_t)1, flags_at = (chain_at + sizeof(ChainCtl) / sizeof(int) + 7) & ~(size_t)7;
     bool good = ok(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) &&
                 dalloc(e, &e->d_desc, 1) && dalloc(e, &e->d_work, P.pairs.size() + e->NG) &&
-                dalloc(e, &e->d_bits, L) && dalloc(e, &e->d_w, L) && dalloc(e, &e->d_osc, L) &&
+                dalloc(e, &e->d_bits, 2 * (size_t)L) && dalloc(e, &e->d_w, L) && dalloc(e, &e->d_osc, L) &&
                 dalloc(e, &e->d_idig, L) && dalloc(e, &e->d_dig, L) && dalloc(e, &e->d_dig2, L) &&
                 dalloc(e, &e->d_eq, 1) && ok(e, cudaMallocHost((void **)&e->h_eq, sizeof(int))) &&
                 dalloc(e, &e->d_slot, (size_t)e->NG * P.R) &&
@@ -276,11 +276,19 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
                 ok(e, cudaMallocHost((void **)&e->h_err, 2 * sizeof(unsigned long long)));
     if (good) {
         std::vector<int64_t> wfix(L), osc(L), idig(L);
+        std::vector<uint8_t> widths(e->lay.bits);  // then TestDesc::segbits
+        widths.resize(2 * (size_t)L);
+        const uint32_t G = (uint32_t)e->G;
         // k / 4H and 1 / R as m 2^e with m in [1/2, 1)
         const double ms = std::frexp((double)k / (4.0 * H), &e->desc.osc_exp);
         const double mi = std::frexp(1.0 / P.R, &e->desc.idig_exp);
-        for (uint32_t j = 0; j < L; j++) {
-            wfix[j] = (int64_t)(wv[j] * 0x1p61);
+        for (uint32_t j = 0, r = 0, c = 0; j < L; j++) {
+            wfix[2 * (c * P.R + r) + j % 2] = (int64_t)(wv[j] * 0x1p61);
+            widths[L + 2 * (c / G * G * P.R + r * G + c % G) + j % 2] = e->lay.bits[j];
+            if (j % 2 && ++c == P.C) {
+                c = 0;
+                r++;
+            }
             const double inv = 1.0 / wv[j];
             osc[j] = fixed_ratio(ms, wv[j], inv);
             idig[j] = fixed_ratio(mi, wv[j], inv);
@@ -296,7 +304,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         std::vector<WorkItem> work;
         for (size_t i = 0; i < P.pairs.size(); i++) work.push_back({0, (int)i});
         for (uint32_t g = 0; g < e->NG; g++) work.push_back({0, (int)g});
-        good = ok(e, cudaMemcpy(e->d_bits, e->lay.bits.data(), L, cudaMemcpyHostToDevice)) &&
+        good = ok(e, cudaMemcpy(e->d_bits, widths.data(), 2 * (size_t)L, cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemcpy(e->d_w, wfix.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemcpy(e->d_osc, osc.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
                ok(e, cudaMemcpy(e->d_idig, idig.data(), L * sizeof(int64_t), cudaMemcpyHostToDevice)) &&
@@ -322,6 +330,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         d.pairs = P.dpairs;
         d.npairs = (int)P.pairs.size();
         d.bits = e->d_bits;
+        d.segbits = e->d_bits + L;
         d.w = e->d_w;
         d.osc = e->d_osc;
         d.idig = e->d_idig;

@@ -19,21 +19,18 @@ __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;
 __device__ __forceinline__ void pdl_leave() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // The walk of a pass kernel over its work list.  What does not depend on the previous kernel is done
-// before pdl_enter: the first item's descriptor and the prefetch of its tables.  The lists and
+// before pdl_enter: the first item's descriptor.  The lists and
 // descriptors are written by copies, which no kernel launched with the attribute overtakes; after a
 // kernel that writes a descriptor the pass is launched without it (LaunchSet::overlap).
-template <class Touch, class Item>
+template <class Item>
 __device__ __forceinline__ void walk_items(const TestDesc *tests, const WorkItem *work, int nwork, int step,
-                                           TestDesc *s_desc, ItemCtl *s_ctl, Touch &&touch_tables, Item &&item) {
+                                           TestDesc *s_desc, ItemCtl *s_ctl, Item &&item) {
     const int first = blockIdx.x;
-    if (first < nwork) {
-        const WorkItem it = work[first];
-        touch_tables(stage_desc(tests, it.test, s_desc, s_ctl), it.unit);
-    }
+    if (first < nwork) stage_desc(tests, work[first].test, s_desc, s_ctl);
     pdl_enter();
     for (int wi = first; wi < nwork; wi += gridDim.x) {
         const WorkItem it = work[wi];
-        if (wi != first) touch_tables(stage_desc(tests, it.test, s_desc, s_ctl), it.unit);
+        if (wi != first) stage_desc(tests, it.test, s_desc, s_ctl);
         if (step < s_desc->count)
             item(*s_desc, it.unit);  // ends with a barrier
         else

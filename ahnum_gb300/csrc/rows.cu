@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_rows(const TestDesc *_
     __shared__ TestDesc s_desc;
     __shared__ ItemCtl s_ctl;
     if (nwork_dev) nwork = *nwork_dev;
-    walk_items(tests, work, nwork, step, &s_desc, &s_ctl, touch_rows, [&](const TestDesc &T, int unit) {
+    walk_items(tests, work, nwork, step, &s_desc, &s_ctl, [&](const TestDesc &T, int unit) {
         rows_item<MUL, GlobalTables>(T, unit, xo ? xo : T.x, MUL ? (yo ? yo : T.y) : nullptr, sm, s_ctl);
     });
 }
