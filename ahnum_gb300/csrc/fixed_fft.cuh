@@ -257,36 +257,46 @@ __device__ __forceinline__ void butterfly(longlong2 *x, const int4 *tw, long lon
 // One stage over 2^LG interleaved sequences, element e of sequence l at (e << LG) + l of the buffers.
 // ld(at, e, l) gives the element (at: its index in the source), st(at, e, l, v) takes the result (at:
 // its index in the destination).  Bit l of `odd` draws the rounding of sequence l (half_of).
-template <int P, int LG, bool INV, bool FIRST, class TAB, class LD, class ST>
+// The loads come first: ld only reads, cook(v, e, l) makes the element of what it read, and pre(e, l)
+// reads what st will need besides.  Read where they are used, the first stage of a column inverse waited
+// for its P loads from L2 one after the other, and the last one for its P scales: at 256 tests of
+// n = 300000 to 700000 the column inverse took 0.133 ms, and 0.101 ms so; the forward 0.096 and 0.089.
+template <int P, int LG, bool INV, bool FIRST, class TAB, class LD, class COOK, class PRE, class ST>
 __device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const int4 *tw, unsigned odd,
-                                          LD &&ld, ST &&st) {
+                                          LD &&ld, COOK &&cook, PRE &&pre, ST &&st) {
     const int np = n / P, total = np << LG;
     for (int i = threadIdx.x; i < total; i += blockDim.x) {
         const int l = i & ((1 << LG) - 1), e = i >> LG;
         const int blk = FIRST ? e : (int)(((unsigned long long)(unsigned)e * magic) >> 32);  // e / span
         const int k = FIRST ? 0 : e - blk * span;
+        const int o = e + blk * (P - 1) * span;
+        decltype(pre(0, 0)) ahead[P];
+#pragma unroll
+        for (int t = 0; t < P; t++) ahead[t] = pre(o + t * span, l);
+        decltype(ld(0, 0, 0)) in[P];
+#pragma unroll
+        for (int t = 0; t < P; t++) in[t] = ld(i + t * total, e + t * np, l);
         longlong2 x[P];
 #pragma unroll
-        for (int t = 0; t < P; t++) x[t] = ld(i + t * total, e + t * np, l);
+        for (int t = 0; t < P; t++) x[t] = cook(in[t], e + t * np, l);
         if constexpr (P > 1) butterfly<P, INV, FIRST, TAB>(x, tw + k * (P - 1), half_of((odd >> l) & 1));
-        const int o = e + blk * (P - 1) * span;
 #pragma unroll
-        for (int t = 0; t < P; t++) st((((o + t * span) << LG) + l), o + t * span, l, x[t]);
+        for (int t = 0; t < P; t++) st((((o + t * span) << LG) + l), o + t * span, l, x[t], ahead[t]);
     }
 }
 
 // The stage of radix p; the last stage of a short transform may have radix 1.
-template <int LG, bool INV, bool FIRST, bool LAST, class TAB, class LD, class ST>
-__device__ __forceinline__ void dispatch_stage(int n, const FftStage &g, const int4 *tw, unsigned odd, LD &&ld, ST &&st) {
+template <int LG, bool INV, bool FIRST, bool LAST, class TAB, class LD, class COOK, class PRE, class ST>
+__device__ __forceinline__ void dispatch_stage(int n, const FftStage &g, const int4 *tw, unsigned odd, LD &&ld, COOK &&cook, PRE &&pre, ST &&st) {
     const int p = g.radix, span = g.span;
     const unsigned magic = g.magic;
     tw += g.off;
 #define KG_STAGE(P)                                                          \
     case P:                                                                  \
-        run_stage<P, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, st);       \
+        run_stage<P, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, cook, pre, st);       \
         break;
     if (p == 4) {
-        run_stage<4, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, st);
+        run_stage<4, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, cook, pre, st);
         return;
     }
     switch (p) {
@@ -295,7 +305,7 @@ __device__ __forceinline__ void dispatch_stage(int n, const FftStage &g, const i
         KG_STAGE(5)
         KG_STAGE(7)
     default:
-        if constexpr (LAST) run_stage<1, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, st);
+        if constexpr (LAST) run_stage<1, LG, INV, FIRST, TAB>(n, span, magic, tw, odd, ld, cook, pre, st);
         break;
     }
 #undef KG_STAGE

@@ -83,18 +83,23 @@ __device__ __forceinline__ int top_exponent(unsigned top) { return (int)(top >> 
 // keeps scales of numbers that are all zero, or far outside what digits can make, in range
 __device__ __forceinline__ int clamp_scale(int s) { return max(-900, min(900, s)); }
 
+struct Nothing {};
+__device__ __forceinline__ Nothing nothing_ahead(int, int) { return {}; }
+__device__ __forceinline__ longlong2 as_read(longlong2 v, int, int) { return v; }
+
 // The whole transform of 2^LG interleaved sequences: the first stage reads first_ld(at, e, l) and
 // writes to `to`, the stages then go back and forth between `to` and `alt`, and the last one
-// calls last_st(dst, at, e, l, v), dst being the buffer it may write to (the value returned).
+// calls last_st(dst, at, e, l, v, last_pre(e, l)), dst being the buffer it may write to (the value
+// returned) and last_pre what it reads from the tables, asked for before the stage's own work.
 // Long transforms are scaled to their largest component once more on the way (FftPlan::renorm,
 // *mid a zeroed word of the block) by 2^shift, set before the last stage.  Ends with a barrier.
-template <int LG, bool INV, class TAB, class LD, class ST>
+template <int LG, bool INV, class TAB, class LD, class COOK, class PRE, class ST>
 __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *tw, longlong2 *to, longlong2 *alt,
-                                                unsigned odd, LD &&first_ld, ST &&last_st, unsigned *mid, int &shift) {
+                                                unsigned odd, LD &&first_ld, COOK &&cook, PRE &&last_pre, ST &&last_st, unsigned *mid, int &shift) {
     const int n = pl.n, last = pl.ns - 1, renorm = pl.renorm;
     shift = 0;
-    dispatch_stage<LG, INV, true, false, TAB>(n, pl.stage[0], tw, odd, first_ld,
-                                         [&](int at, int, int, longlong2 v) { to[at] = v; });
+    dispatch_stage<LG, INV, true, false, TAB>(n, pl.stage[0], tw, odd, first_ld, cook, nothing_ahead,
+                                         [&](int at, int, int, longlong2 v, Nothing) { to[at] = v; });
     __syncthreads();
     for (int i = 1; i < last; i++) {
         odd = ~odd;
@@ -106,8 +111,9 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
             const bool track = i + 1 == renorm;
             unsigned mag = 0;
             dispatch_stage<LG, INV, false, false, TAB>(
-                n, pl.stage[i], tw, odd, [&](int at, int, int) { return cshl(from[at], sh); },
-                [&](int at, int, int, longlong2 v) {
+                n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; },
+                [&](longlong2 v, int, int) { return cshl(v, sh); }, nothing_ahead,
+                [&](int at, int, int, longlong2 v, Nothing) {
                     to[at] = v;
                     mag |= mag32(v);
                 });
@@ -115,13 +121,13 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
             __syncthreads();
             if (track) shift = 29 - bit_length(*mid);  // components below 2^61
         } else {
-            dispatch_stage<LG, INV, false, false, TAB>(n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; },
-                                                  [&](int at, int, int, longlong2 v) { to[at] = v; });
+            dispatch_stage<LG, INV, false, false, TAB>(n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; }, as_read, nothing_ahead,
+                                                  [&](int at, int, int, longlong2 v, Nothing) { to[at] = v; });
             __syncthreads();
         }
     }
-    dispatch_stage<LG, INV, false, true, TAB>(n, pl.stage[last], tw, ~odd, [&](int at, int, int) { return to[at]; },
-                                         [&](int at, int e, int l, longlong2 v) { last_st(alt, at, e, l, v); });
+    dispatch_stage<LG, INV, false, true, TAB>(n, pl.stage[last], tw, ~odd, [&](int at, int, int) { return to[at]; }, as_read, last_pre,
+                                         [&](int at, int e, int l, longlong2 v, auto p) { last_st(alt, at, e, l, v, p); });
     __syncthreads();
     return alt;
 }
@@ -211,11 +217,10 @@ __device__ __forceinline__ longlong2 *rows_forward(const TestDesc &T, int2 pr, c
     int shift;
     longlong2 *out = transform<1, false, TAB>(
         pl, T.twr, other, raw, odd,
-        [&](int at, int, int) {
-            const longlong2 d = raw[at];
-            return make_longlong2(to_fixed(d.x, s), to_fixed(d.y, s));
-        },
-        [&](longlong2 *dst, int at, int, int, longlong2 v) {
+        [&](int at, int, int) { return raw[at]; },
+        [&](longlong2 d, int, int) { return make_longlong2(to_fixed(d.x, s), to_fixed(d.y, s)); },
+        nothing_ahead,
+        [&](longlong2 *dst, int at, int, int, longlong2 v, Nothing) {
             dst[at] = v;
             m |= mag32(v);
         },
@@ -282,8 +287,9 @@ __device__ __forceinline__ void rows_item(const TestDesc &T, int unit, double2 *
     mag = 0;
     int shift;
     transform<1, true, TAB>(
-        pl, T.twr, other, X, odd, [&](int at, int, int) { return cshift(X[at], ns); },
-        [&](longlong2 *, int, int e, int l, longlong2 v) {
+        pl, T.twr, other, X, odd, [&](int at, int, int) { return X[at]; },
+        [&](longlong2 v, int, int) { return cshift(v, ns); }, nothing_ahead,
+        [&](longlong2 *, int, int e, int l, longlong2 v, Nothing) {
             if (l && self) return;
             (l ? ob : oa)[e] = v;
             mag |= mag32(v);
@@ -484,6 +490,13 @@ __device__ __forceinline__ void segment_carries(const TestDesc &T, int g, const 
     }
 }
 
+// What the first stage of a column inverse reads: a component pair, its twiddle, its row's exponent.
+struct TurnedIn {
+    longlong2 v;
+    int4 w;
+    int up;
+};
+
 // One column group of one test, first half of the column pass.  Ends with a barrier after its
 // last global write.
 template <int LG, class TAB>
@@ -504,14 +517,13 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
     unsigned err = 0, big = 0;
     longlong2 *digits = transform<LG, true, TAB>(
         pl, T.twc, sm, sm + (T.R << LG), odd,
-        [&](int, int k, int l) {
-            const int e = k * C + l;
-            return cmul(cshift(__ldcg(&x[e]), __ldcg(&rexp[k]) + se), conj_tw(TAB::load(&t4[k * T.pitch + l])),
-                        half_of(parity(k) ^ ((odd >> l) & 1)));
+        [&](int, int k, int l) { return TurnedIn{__ldcg(&x[k * C + l]), TAB::load(&t4[k * T.pitch + l]), __ldcg(&rexp[k])}; },
+        [&](const TurnedIn &in, int k, int l) {
+            return cmul(cshift(in.v, in.up + se), conj_tw(in.w), half_of(parity(k) ^ ((odd >> l) & 1)));
         },
-        [&](longlong2 *dst, int, int r, int l, longlong2 v) {
+        [&](int r, int l) { return TAB::load(reinterpret_cast<const longlong2 *>(osc + 2 * (r * T.pitch + l))); },
+        [&](longlong2 *dst, int, int r, int l, longlong2 v, longlong2 o) {
             // unweight, scale and round
-            const longlong2 o = TAB::load(reinterpret_cast<const longlong2 *>(osc + 2 * (r * T.pitch + l)));
             const int m = min((unsigned)(n + shift), 95u);
             int fx, fy;
             v.x = scale_round(v.x, o.x, m, fx);
@@ -593,10 +605,11 @@ __device__ __forceinline__ void col_forward_item(const TestDesc &T, int g, doubl
     double2 *xg = x + (g << LG);
     const int4 *t4 = T.t4 + (g << LG);
     transform<LG, false, TAB>(
-        pl, T.twc, sm + (T.R << LG), sm, odd, [&](int, int r, int l) { return sm[turned<LG>(r, l)]; },
-        [&](longlong2 *, int, int k, int l, longlong2 v) {
+        pl, T.twc, sm + (T.R << LG), sm, odd, [&](int, int r, int l) { return sm[turned<LG>(r, l)]; }, as_read,
+        [&](int k, int l) { return TAB::load(&t4[k * T.pitch + l]); },
+        [&](longlong2 *, int, int k, int l, longlong2 v, int4 w) {
             const int e = k * C + l;
-            const longlong2 z = cmul(v, TAB::load(&t4[k * T.pitch + l]), half_of(parity(k) ^ ((odd >> l) & 1)));
+            const longlong2 z = cmul(v, w, half_of(parity(k) ^ ((odd >> l) & 1)));
             xg[e] = make_double2(from_fixed(z.x, ex - up), from_fixed(z.y, ex - up));
         },
         &ctl.mid[0], up);
@@ -625,14 +638,14 @@ __device__ __forceinline__ void col_digits_item(const TestDesc &T, int g, const 
     int shift;
     transform<LG, true, TAB>(
         pl, T.twc, sm + (R << LG), sm, odd,
-        [&](int at, int k, int l) {
-            const longlong2 d = sm[at];
-            return cmul(make_longlong2(to_fixed(d.x, se), to_fixed(d.y, se)), conj_tw(TAB::load(&t4[k * T.pitch + l])),
+        [&](int at, int k, int l) { return TurnedIn{sm[at], TAB::load(&t4[k * T.pitch + l]), 0}; },
+        [&](const TurnedIn &in, int k, int l) {
+            return cmul(make_longlong2(to_fixed(in.v.x, se), to_fixed(in.v.y, se)), conj_tw(in.w),
                         half_of(parity(k) ^ ((odd >> l) & 1)));
         },
-        [&](longlong2 *, int, int r, int l, longlong2 v) {
+        [&](int r, int l) { return __ldg(reinterpret_cast<const longlong2 *>(T.idig + 2 * (r * C + (g << LG) + l))); },
+        [&](longlong2 *, int, int r, int l, longlong2 v, longlong2 o) {
             const int j = 2 * (r * C + (g << LG) + l), m = n + shift;
-            const longlong2 o = __ldg(reinterpret_cast<const longlong2 *>(T.idig + j));
             int f;
             dig[j] = shift_by(scale_round(v.x, o.x, max(0, min(m, 95)), f), max(0, -m));
             dig[j + 1] = shift_by(scale_round(v.y, o.y, max(0, min(m, 95)), f), max(0, -m));
