@@ -236,17 +236,17 @@ struct AnyTables {
 // One radix-P butterfly of a stage with twiddle records w^t, t = 1..P-1 (tw).  UNIT: the stage of
 // span 1, whose twiddles are 1.  A twiddled butterfly of radix 3, 4, 5 or 7 divides by 4, the others
 // do not scale.
-template <int P, bool INV, bool UNIT, class TAB>
+template <int P, bool INV, bool UNIT>
 __device__ __forceinline__ void butterfly(longlong2 *x, const int4 *tw, long long half) {
     if constexpr (!UNIT) {
         if constexpr (P == 2) {
-            const int4 w = TAB::load(tw);  // unscaled
+            const int4 w = tw[0];  // unscaled
             x[1] = cmul4(x[1], INV ? conj_tw(w) : w);
         } else {
             x[0] = quarter(x[0], half);
 #pragma unroll
             for (int t = 1; t < P; t++) {
-                const int4 w = TAB::load(tw + t - 1);
+                const int4 w = tw[t - 1];
                 x[t] = cmul(x[t], INV ? conj_tw(w) : w, half);
             }
         }
@@ -260,7 +260,7 @@ __device__ __forceinline__ void butterfly(longlong2 *x, const int4 *tw, long lon
 // The loads come first: ld only reads, cook(v, e, l) makes the element of what it read, and pre(e, l)
 // reads what st will need besides.  Read where they are used, the first stage of a column inverse waited
 // for its P loads from L2 one after the other, and the last one for its P scales: at 256 tests of
-// n = 300000 to 700000 the column inverse took 0.133 ms, and 0.101 ms so; the forward 0.096 and 0.089.
+// n = 300000 to 700000 the column inverse took 0.133 ms, and 0.100 ms so; the forward 0.096 and 0.087.
 template <int P, int LG, bool INV, bool FIRST, class TAB, class LD, class COOK, class PRE, class ST>
 __device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const int4 *tw, unsigned odd,
                                           LD &&ld, COOK &&cook, PRE &&pre, ST &&st) {
@@ -270,6 +270,11 @@ __device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const
         const int blk = FIRST ? e : (int)(((unsigned long long)(unsigned)e * magic) >> 32);  // e / span
         const int k = FIRST ? 0 : e - blk * span;
         const int o = e + blk * (P - 1) * span;
+        int4 w[FIRST || P == 1 ? 1 : P - 1];
+        if constexpr (!FIRST) {
+#pragma unroll
+            for (int t = 0; t < P - 1; t++) w[t] = TAB::load(tw + k * (P - 1) + t);
+        }
         decltype(pre(0, 0)) ahead[P];
 #pragma unroll
         for (int t = 0; t < P; t++) ahead[t] = pre(o + t * span, l);
@@ -279,7 +284,7 @@ __device__ __forceinline__ void run_stage(int n, int span, unsigned magic, const
         longlong2 x[P];
 #pragma unroll
         for (int t = 0; t < P; t++) x[t] = cook(in[t], e + t * np, l);
-        if constexpr (P > 1) butterfly<P, INV, FIRST, TAB>(x, tw + k * (P - 1), half_of((odd >> l) & 1));
+        if constexpr (P > 1) butterfly<P, INV, FIRST>(x, w, half_of((odd >> l) & 1));
 #pragma unroll
         for (int t = 0; t < P; t++) st((((o + t * span) << LG) + l), o + t * span, l, x[t], ahead[t]);
     }

@@ -550,6 +550,11 @@ __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool us
     constexpr int LG = G == 8 ? 3 : G == 4 ? 2 : 1;
     // absorb the carry-in into the segment's first digits (the last digit takes any rest), reweight
     for (int r = threadIdx.x; r < R; r += blockDim.x) {
+        const SegWidths<G> bw = load_segment_widths<G, TAB>(T.segbits, 2 * G * (g * R + r));
+        long long cy = use_slots ? __ldcg(&T.slot[g * R + r]) : 0;
+        const longlong2 *wv = reinterpret_cast<const longlong2 *>(T.w) + g * G * R + r;
+        constexpr int kEarly = G / 2;
+        longlong2 we[kEarly];
         long long d[2 * G];
         const longlong2 *src = reinterpret_cast<const longlong2 *>(T.dig) + (use_slots ? g * G * R + r : r * T.C + g * G);
         const int column = use_slots ? R : 1;
@@ -559,8 +564,8 @@ __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool us
             d[2 * l] = p.x;
             d[2 * l + 1] = p.y;
         }
-        long long cy = use_slots ? __ldcg(&T.slot[g * R + r]) : 0;
-        const SegWidths<G> bw = load_segment_widths<G, TAB>(T.segbits, 2 * G * (g * R + r));
+#pragma unroll
+        for (int l = 0; l < kEarly; l++) we[l] = TAB::load(wv + l * R);
 #pragma unroll
         for (int i = 0; i < 2 * G - 1; i++) {
             if (cy) {
@@ -572,10 +577,9 @@ __device__ __forceinline__ void absorb_carries(const TestDesc &T, int g, bool us
             }
         }
         d[2 * G - 1] += cy;
-        const longlong2 *wv = reinterpret_cast<const longlong2 *>(T.w) + g * G * R + r;
 #pragma unroll
         for (int l = 0; l < G; l++) {
-            const longlong2 w = TAB::load(wv + l * R);
+            const longlong2 w = l < kEarly ? we[l < kEarly ? l : 0] : TAB::load(wv + l * R);
             const long long a = shift_by(d[2 * l], shift), b = shift_by(d[2 * l + 1], shift);
             Acc x, y;
             x.mac(hi32(a), lo32(a), hi32(w.x), lo32(w.x));
