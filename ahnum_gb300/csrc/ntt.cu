@@ -193,21 +193,25 @@ struct Fold {
     uint64_t q, lo, r0, r1;  // T = E >> n = q k + r: q joins word 0, r 2^n the words WN0 and WN0 + 1
 };
 
+// NUMBER: the product is the W words at D.pw, without segment carries (a number, to be divided by 2^n).
+template <bool NUMBER>
 __device__ __forceinline__ uint64_t product_word(const Desc &D, uint32_t j) {
     uint64_t v = D.pw[j];
-    if ((j & 7) < 2 && j >= 8) {
+    if (!NUMBER && (j & 7) < 2 && j >= 8) {
         const ulonglong2 c = D.seg[(j >> 3) - 1];  // < 2^(w+20): its low word and the rest
         v += (j & 7) == 0 ? c.x & ((1ull << D.w) - 1) : (c.x >> D.w) | (c.y << (64 - D.w));
     }
     return v;
 }
 
+template <bool NUMBER>
 __device__ __forceinline__ u128 reduced_word(const Desc &D, int j, const uint64_t *addend) {
     if (j < 0 || j > (int)D.W) return 0;
+    const uint32_t len = NUMBER ? D.W : D.NP;
     const uint64_t low = (1ull << D.BN0) - 1;
     const uint32_t s = D.WN0 + j;
-    const uint64_t v0 = s < D.NP ? product_word(D, s) : 0, v1 = D.BN0 && s + 1 < D.NP ? product_word(D, s + 1) : 0;
-    const uint64_t a = j < (int)D.WN0 ? product_word(D, j) : j == (int)D.WN0 ? product_word(D, j) & low : 0;
+    const uint64_t v0 = s < len ? product_word<NUMBER>(D, s) : 0, v1 = D.BN0 && s + 1 < len ? product_word<NUMBER>(D, s + 1) : 0;
+    const uint64_t a = j < (int)D.WN0 ? product_word<NUMBER>(D, j) : j == (int)D.WN0 ? product_word<NUMBER>(D, j) & low : 0;
     u128 e = (u128)D.k * a + (v0 >> D.BN0) + ((v1 & low) << (D.w - D.BN0));
     if (addend && j < (int)D.W) e += addend[j];
     return e;
@@ -229,10 +233,11 @@ __device__ __forceinline__ uint64_t two_carries(u128 e, uint32_t w, int lane, in
 }
 
 // One warp: T = E >> n from the words WN0 .. W of E, its quotient and remainder by k.
+template <bool NUMBER>
 __device__ __forceinline__ void fold_of(const Desc &D, const uint64_t *addend, Fold *f) {
     const int lane = threadIdx.x & 31;
     uint32_t c1, c2;
-    const u128 e = reduced_word(D, (int)D.WN0 - 2 + lane, addend);
+    const u128 e = reduced_word<NUMBER>(D, (int)D.WN0 - 2 + lane, addend);
     const uint64_t x = two_carries(e, D.w, lane, 32, 0, 0, &c1, &c2);  // exact from lane 2 on: word WN0
     const uint64_t xn = __shfl_sync(0xffffffffu, x, 2);
     u128 T = xn >> D.BN0;
@@ -246,8 +251,10 @@ __device__ __forceinline__ void fold_of(const Desc &D, const uint64_t *addend, F
         else T += (u128)v << sh;
     }
     if (lane == 0) {
-        const ulonglong2 out = D.seg[(D.NP >> 3) - 1];
-        if (out.x | out.y) bad |= 1;
+        if (!NUMBER) {
+            const ulonglong2 out = D.seg[(D.NP >> 3) - 1];
+            if (out.x | out.y) bad |= 1;
+        }
         uint64_t q, r0;
         if ((T >> 64) == 0) {  // always for k < 2^30 and a number below N: T < 2^(2 log2 k + 3)
             const uint64_t t64 = (uint64_t)T;
@@ -271,10 +278,10 @@ __device__ __forceinline__ void fold_of(const Desc &D, const uint64_t *addend, F
 
 // Word j = r C + 8 g + l of E, by lane l of the eight that hold the row.
 __device__ __forceinline__ uint64_t folded_word(const Desc &D, int j, int l, const uint64_t *addend, const Fold &f) {
-    u128 e = reduced_word(D, j, addend);
+    u128 e = reduced_word<false>(D, j, addend);
     if (j == 0) e += f.q;
     // the two words before the eight: lanes 6 and 7 evaluate them besides their own
-    const u128 h = l >= 6 ? reduced_word(D, j - 8, addend) : 0;
+    const u128 h = l >= 6 ? reduced_word<false>(D, j - 8, addend) : 0;
     uint32_t c1, c2, h1, h2;
     (void)two_carries(h, D.w, l, 8, 0, 0, &h1, &h2);
     const uint32_t c1b = __shfl_sync(0xffffffffu, h1, 7, 8), c2b = __shfl_sync(0xffffffffu, h2, 7, 8);
@@ -295,7 +302,7 @@ __device__ __forceinline__ void col_fwd_item(uint32_t *sm, const Desc &D, int g,
         bool mine = g == 0;
         for (uint32_t j = D.WN0; j < D.W; j++) mine |= (int)((j & (C - 1)) >> 3) == g;
         if (mine) {
-            if (threadIdx.x < 32) fold_of(D, src, &f);
+            if (threadIdx.x < 32) fold_of<false>(D, src, &f);
             __syncthreads();
         }
     }
@@ -766,13 +773,80 @@ __global__ void __launch_bounds__(kReduceThreads) kn_reduce(const Desc *descs, c
     }
 }
 
+// The status of the members that have one.
+__global__ void kn_any_status(const Desc *descs, int n, int *any) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && *descs[i].status) atomicOr(any, *descs[i].status);
+}
+
+// num 2^-n as 64-bit limbs, a block for each kLimbThreads of them, by the same two steps of carries as
+// Fold.  A word of exactly 2^w (a carry into 2^w - 1) would have to ripple: then *ripple is set and
+// the caller takes the exact way, kn_reduce<true> and kn_limbs.
+constexpr int kLimbThreads = 128;
+constexpr int kLimbWords = kLimbThreads * 64 / 33 + 6;  // w >= 33: the block's words and the two before
+
+__global__ void __launch_bounds__(kLimbThreads) kn_number_limbs(const Desc *desc, const uint64_t *num, uint64_t *limbs,
+                                                               uint32_t nlimbs, unsigned long long *ripple) {
+    __shared__ Desc s_desc;
+    __shared__ Fold s_fold;
+    __shared__ uint64_t s_low[kLimbWords];
+    __shared__ uint32_t s_carry[kLimbWords];
+    for (int i = threadIdx.x; i < (int)(sizeof(Desc) / 8); i += blockDim.x)
+        reinterpret_cast<uint64_t *>(&s_desc)[i] = reinterpret_cast<const uint64_t *>(desc)[i];
+    __syncthreads();
+    if (threadIdx.x == 0) s_desc.pw = const_cast<uint64_t *>(num);
+    __syncthreads();
+    const Desc &D = s_desc;
+    const uint32_t w = D.w, first = blockIdx.x * kLimbThreads, last = min(nlimbs, first + kLimbThreads);  // limbs
+    const uint64_t M = (1ull << w) - 1;
+    const int j0 = (int)(64ull * first / w) - 2, j1 = (int)((64ull * last - 1) / w);  // words, two before the first
+    if (j0 <= 0 || j1 >= (int)D.WN0) {
+        if (threadIdx.x < 32) fold_of<true>(D, nullptr, &s_fold);
+        __syncthreads();
+    }
+    for (int j = j0 + (int)threadIdx.x; j <= j1; j += blockDim.x) {
+        u128 e = reduced_word<true>(D, j, nullptr);
+        if (j == 0) e += s_fold.q;
+        s_low[j - j0] = (uint64_t)e & M;
+        s_carry[j - j0] = (uint32_t)(e >> w);
+    }
+    __syncthreads();
+    const auto word = [&](int j) -> uint64_t {
+        if (j >= (int)D.W) return 0;
+        if (j >= (int)D.WN0) return j == (int)D.WN0 ? s_fold.lo + s_fold.r0 : j == (int)D.WN0 + 1 ? s_fold.r1 : 0;
+        const int i = j - j0;  // >= 2
+        const uint64_t before = s_low[i - 1] + s_carry[i - 2], v = s_low[i] + s_carry[i - 1];
+        return (v & M) + (before >> w);
+    };
+    const uint32_t i = first + threadIdx.x;
+    if (i >= last) return;
+    const uint64_t bit = 64ull * i;
+    int j = (int)(bit / w);
+    uint32_t have = w - (uint32_t)(bit % w);
+    uint64_t x = word(j), most = x, v = x >> (w - have);
+    for (j++; have < 64; j++, have += w) {
+        x = word(j);
+        most |= x;
+        v |= x << have;
+    }
+    limbs[i] = v;
+    if (most > M) atomicOr(ripple, 1ull);
+}
+
+// The status and *ripple, which is cleared, after a number's limbs.
+__global__ void kn_limbs_end(const int *status, unsigned long long *ripple, uint64_t *out) {
+    pdl_enter();
+    *out = (uint64_t)(uint32_t)*status | (uint64_t)*ripple << 32;
+    *ripple = 0;
+}
+
 // The words X (below 2^w each) as 64-bit limbs, and the status word after the last one.
 __global__ void kn_limbs(const uint64_t *X, uint32_t W, uint32_t w, uint64_t *limbs, uint32_t nlimbs, const int *status) {
     pdl_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > nlimbs) return;
     if (i == nlimbs) {
-        limbs[i] = (uint64_t)(int64_t)*status;
+        limbs[i] = (uint64_t)(uint32_t)*status;
         return;
     }
     const uint64_t bit = 64ull * i;
@@ -1009,7 +1083,8 @@ struct kn_engine : kn::NumLayout {
     ulonglong2 *d_seg = nullptr;
     uint64_t *d_pw = nullptr;
     uint64_t *d_addend = nullptr;
-    uint64_t *d_out = nullptr;  // W words, then the limbs and the status of the number being read
+    // the number being read: W words, its limbs and status, and a word of kn_number_limbs
+    uint64_t *d_out = nullptr;
     std::mutex out_mu;          // held from the first write to d_out until it is copied
     int64_t addend_c = 0;
     bool addend_ok = false;
@@ -1281,7 +1356,8 @@ kn_engine *kn_engine_new(uint64_t k, uint64_t n, int device) {
               kok(e, cudaMalloc((void **)&e->d_seg, (size_t)(NP / kG) * sizeof(ulonglong2))) &&
               kok(e, cudaMalloc((void **)&e->d_pw, (size_t)NP * 8)) &&
               kok(e, cudaMalloc((void **)&e->d_addend, (size_t)e->W * 8)) &&
-              kok(e, cudaMalloc((void **)&e->d_out, ((size_t)e->W + e->nlimbs + 1) * 8)) &&
+              kok(e, cudaMalloc((void **)&e->d_out, ((size_t)e->W + e->nlimbs + 2) * 8)) &&
+              kok(e, cudaMemset(e->d_out, 0, ((size_t)e->W + e->nlimbs + 2) * 8)) &&
               kok(e, cudaMalloc((void **)&e->d_status, sizeof(int))) &&
               kok(e, cudaMalloc((void **)&e->d_cols, (C / kG) * sizeof(int2))) &&
               kok(e, cudaMalloc((void **)&e->d_rows, R * sizeof(int2))) &&
@@ -1388,7 +1464,8 @@ int kn_set_limbs(kn_engine *e, uint64_t *x, const uint64_t *limbs) {
 
 // x~ 2^-n mod N by the product's reduction and the repacking on the GPU; a value of N or more (a
 // number equal to N, or one that was never reduced) is finished on the host.  On GB300, n = 300000 to
-// 700000: 55 us a number, half of it the reduction's one block; 112 us with the arithmetic on the host.
+// 700000: 39 us a number, 55 us through kn_reduce's one block, 112 us with the arithmetic
+// on the host.
 int kn_get_limbs(kn_engine *e, const uint64_t *x, uint64_t *limbs) {
     if (!e || e->err) return -1;
     std::vector<uint64_t> v(e->nlimbs + 1);
@@ -1396,13 +1473,26 @@ int kn_get_limbs(kn_engine *e, const uint64_t *x, uint64_t *limbs) {
     {
         std::lock_guard<std::mutex> lock(e->out_mu);
         uint64_t *out = e->d_out + e->W;
-        const int grid = (int)((e->nlimbs + 1 + 255) / 256);
-        launch(false, kn_reduce<true>, 1, kReduceThreads, 0, e->stream, e->d_desc, e->d_test, e->d_out, nullptr, x);
-        launch(true, kn_limbs, grid, 256, 0, e->stream, e->d_out, e->W, e->w, out, (uint32_t)e->nlimbs, e->d_status);
-        if (!kok(e, cudaGetLastError()) ||
-            !kok(e, cudaMemcpyAsync(v.data(), out, v.size() * 8, cudaMemcpyDeviceToHost, e->stream)) ||
-            !kok(e, cudaStreamSynchronize(e->stream)))
-            return -1;
+        const uint32_t nl = (uint32_t)e->nlimbs;
+        const auto read = [&] {
+            return kok(e, cudaGetLastError()) &&
+                   kok(e, cudaMemcpyAsync(v.data(), out, v.size() * 8, cudaMemcpyDeviceToHost, e->stream)) &&
+                   kok(e, cudaStreamSynchronize(e->stream));
+        };
+        bool exact = !e->lazy;
+        if (!exact) {
+            unsigned long long *ripple = reinterpret_cast<unsigned long long *>(out + nl + 1);
+            launch(false, kn_number_limbs, (int)((nl + kLimbThreads - 1) / kLimbThreads), kLimbThreads, 0, e->stream, e->d_desc, x, out,
+                   nl, ripple);
+            launch(true, kn_limbs_end, 1, 1, 0, e->stream, e->d_status, ripple, out + nl);
+            if (!read()) return -1;
+            exact = v.back() >> 32;
+        }
+        if (exact) {
+            launch(false, kn_reduce<true>, 1, kReduceThreads, 0, e->stream, e->d_desc, e->d_test, e->d_out, nullptr, x);
+            launch(true, kn_limbs, (int)((nl + 1 + 255) / 256), 256, 0, e->stream, e->d_out, e->W, e->w, out, nl, e->d_status);
+            if (!read()) return -1;
+        }
     }
     if (v.back()) {
         e->err = -100 - (int)v.back();
@@ -1571,7 +1661,7 @@ bool group_build(kn_group *g) {
     bool ok = gok(g, cudaMalloc((void **)&g->d_desc, m * sizeof(Desc))) &&
               gok(g, cudaMalloc((void **)&g->d_cols, cols.size() * sizeof(int2))) &&
               gok(g, cudaMalloc((void **)&g->d_rows, rows.size() * sizeof(int2))) &&
-              gok(g, cudaMalloc((void **)&g->d_tests, m * sizeof(int))) &&
+              gok(g, cudaMalloc((void **)&g->d_tests, (m + 1) * sizeof(int))) &&
               gok(g, cudaMemcpy(g->d_desc, descs.data(), m * sizeof(Desc), cudaMemcpyHostToDevice)) &&
               gok(g, cudaMemcpy(g->d_cols, cols.data(), cols.size() * sizeof(int2), cudaMemcpyHostToDevice)) &&
               gok(g, cudaMemcpy(g->d_rows, rows.data(), rows.size() * sizeof(int2), cudaMemcpyHostToDevice)) &&
@@ -1662,11 +1752,13 @@ bool group_prepare(kn_group *g) {
 
 // sticky device-side status of every member (a carry that did not settle)
 void group_check_status(kn_group *g) {
-    for (kn_engine *e : g->eng) {
-        int st = 0;
-        cudaMemcpy(&st, e->d_status, sizeof st, cudaMemcpyDeviceToHost);
-        if (st) g->err = -100 - st;
-    }
+    int st = 0, *any = g->d_tests + g->ntests;
+    cudaMemsetAsync(any, 0, sizeof st, g->stream);
+    launch(false, kn_any_status, (g->ntests + 127) / 128, 128, 0, g->stream, g->d_desc, g->ntests, any);
+    if (!gok(g, cudaGetLastError()) || !gok(g, cudaMemcpyAsync(&st, any, sizeof st, cudaMemcpyDeviceToHost, g->stream)) ||
+        !gok(g, cudaStreamSynchronize(g->stream)))
+        return;
+    if (st) g->err = -100 - st;
 }
 
 }  // namespace

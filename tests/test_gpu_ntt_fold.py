@@ -100,3 +100,25 @@ def test_group_equals_python(streams):
             a = (C.c_uint64 * g.lib.kn_limbs(e))()
             assert g.lib.kn_get_limbs(e, x, a) == 0
             assert int.from_bytes(bytes(a), "little") == _chain(3, k, n, 20, 0)
+
+
+@pytest.mark.parametrize("n,j", [(1000, 4), (20000, 9), (20000, 150), (369717, 5000), (600000, 7)])
+def test_carry_through_a_full_word_reads_right(n, j):
+    """a number whose words meet a carry into 2^w - 1 when it leaves the Montgomery form: 3 A with the
+    words of A chosen so"""
+    k = 3
+    e = _Engine(k, n)
+    try:
+        w = e.lib.kn_word_bits(e.e)
+        assert (j + 2) * w < n
+        full, inv = (1 << w) - 1, pow(3, -1, 1 << w)
+        a0 = full                                     # 3 a0: a carry of 2
+        a1 = full * inv % (1 << w)                    # 3 a1 = 2^w - 1 (mod 2^w)
+        a2 = (full - (3 * a1 >> w)) * inv % (1 << w)  # with a1's carry the next word is full
+        a = (a0 << (w * (j - 1))) + (a1 << (w * j)) + (a2 << (w * (j + 1)))
+        e.set(3 * a)
+        assert e.get() == 3 * a
+        assert e.lib.kn_square(e.e, e.x, 2) == 0
+        assert e.get() == _chain(3 * a, k, n, 2, 0)
+    finally:
+        e.close()
