@@ -93,8 +93,7 @@ struct kc_batch {
     cudaGraphExec_t graph = nullptr;
     size_t graph_row_smem = 0, graph_col_smem = 0;
     uint32_t graph_B = 0;
-    int grid = 0;
-    int threads = 128;  // block size of the pass kernels
+    int threads = 0;  // block size of the pass kernels (0: block_threads)
     bool persistent = false;      // squaring blocks as the persistent kernel k_squarings
     bool stagger = false;         // first rounds of 1..M blocks by admission order (kc_batch_stagger_checks)
     uint64_t admitted = 0;        // Fermat slots admitted so far
@@ -164,6 +163,17 @@ bool has_narrow(const kc_batch *b) {
     return false;
 }
 
+// Block size of the pass kernels: 128 threads, so that 6 CTAs share an SM with the registers of 3 of
+// 256, and a short transform's stages fill them.  Where the longest item's buffers leave room for
+// fewer than 4 CTAs, 256, or the SM would hold less than 512 threads.  Measured on GB300, ms per
+// squaring of the batch with 128 and 256 threads: the benchmark's 256 tests (36 KB) 0.299 and 0.415,
+// 64 of them 0.078 and 0.106; served mixes with FFT lengths to 294912 (66 KB), 16 tests 0.065 and
+// 0.061, 48 tests 0.169 and 0.155.
+static int block_threads(size_t row_lane, size_t col_smem) {
+    constexpr size_t kSm = 228 * 1024, kBesides = 1024 + 704;  // an SM's shared memory; a CTA's own
+    return kSm / (std::max(row_lane * 4, col_smem) + kBesides) < 4 ? 256 : 128;
+}
+
 LaunchSet launch_set(kc_batch *b, const kc_batch::Lists &l, size_t row_lane, size_t col_smem) {
     LaunchSet s;
     s.stream = b->stream;
@@ -177,9 +187,8 @@ LaunchSet launch_set(kc_batch *b, const kc_batch::Lists &l, size_t row_lane, siz
     s.narrow = has_narrow(b);
     s.cols4 = l.d_cols + l.cap_cols;
     s.ncols4_dev = l.d_cnt + 2;
-    s.grid_rows = b->grid;
-    s.grid_cols = b->grid;
-    s.threads = b->threads;
+    s.threads = b->threads ? b->threads : block_threads(row_lane, col_smem);
+    s.grid_rows = s.grid_cols = b->nsm * (kThreads * kMinBlocks / s.threads);
     s.row_smem_per_lane = row_lane;
     s.col_smem = col_smem;
     return s;
@@ -474,11 +483,12 @@ bool fill_lists(kc_batch *b, kc_batch::Lists &l, const std::vector<Entry> &ents)
 // launch tails and low-occupancy passes.  Measured on GB300, ms per squaring of the batch:
 //
 //   tests (workload)     persistent  per pass  2 parts  3 parts  4 parts
-//   32 (benchmark's)       0.159      0.148     0.137    0.132    0.129
-//   64                     0.262      0.287     0.231    0.230    0.230
-//   256                    0.906      1.010     0.893    0.892    0.895
-//   16 (served mix)        0.233      0.229     0.220    0.213    0.213
-//   48                     0.541      0.495     0.429    0.422    0.421
+//   32 (benchmark's)       0.045      0.051     0.043    0.043    0.046
+//   64                     0.086      0.096     0.078    0.078    0.078
+//   128                    0.181      0.177     0.154    0.159    0.158
+//   256                    0.345      0.333     0.299    0.299    0.300
+//   16 (served mix)        0.071      0.073     0.065    0.065    0.069
+//   48                     0.210      0.195     0.166    0.169    0.170
 //
 // So a block of two or more slots is split in three parts (KITE_GB300_BATCH_SPLIT=P picks P, 1
 // keeps one stream), and the persistent kernel runs only when KITE_GB300_BATCH_PERSISTENT=1
@@ -580,13 +590,8 @@ kc_batch *kc_batch_new(int device, uint32_t gerbicz_block, uint32_t gerbicz_bloc
     cudaMemGetInfo(&fr, &tot);
     b->budget = mem_budget ? mem_budget : fr / 10 * 8;
     cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, device);
-    // Block size of the pass kernels: 128 threads, so that 8 CTAs share an SM with the register
-    // budget (64 per thread) of 4 CTAs of 256.  Measured on GB300 over the 256-test workload:
-    // 1.034 s per 1000-squaring block at 128 threads, 1.103 s at 256 and 1.103 s at 64.
-    // KITE_GB300_BATCH_THREADS=256 selects the larger blocks.
-    b->threads = 128;
+    // KITE_GB300_BATCH_THREADS=128 or 256 overrides block_threads
     if (const char *t = getenv("KITE_GB300_BATCH_THREADS")) b->threads = atoi(t) == 256 ? 256 : 128;
-    b->grid = b->nsm * (kThreads * kMinBlocks / b->threads);
     // A Gerbicz block's squarings run as pass launches in parts on several streams (BlockForm);
     // KITE_GB300_BATCH_PERSISTENT=1 runs them as persistent launches of k_squarings instead
     // (steps_per_launch squarings each).
