@@ -2,10 +2,10 @@
 // over shared memory that the row and column passes run.
 //
 // Why fixed point.  GB300 issues an FP64 instruction once per 64-76 clocks per SM sub-partition,
-// but a 64-bit integer add every clock and a 32 x 32 -> 64-bit multiply-add every two (measured
-// with dependent chains at full occupancy).  A complex product of 64-bit fixed-point numbers is
-// 12 multiply-adds and a few adds, about 32 issue clocks, where its FP64 form costs about 280; a
-// complex add costs 2 instead of about 150.  The squaring was bound by the FP64 pipe (102 FP64
+// but a 64-bit integer add every two and a 32 x 32 -> 64-bit multiply every four (measured with
+// dependent chains at full occupancy).  A complex product of 64-bit fixed-point numbers is
+// 12 multiplies and as many adds, about 65 issue clocks, where its FP64 form costs about 280; a
+// complex add costs 4 instead of about 150.  The squaring was bound by the FP64 pipe (102 FP64
 // instructions per point), so the transforms run in integers, and at no loss of precision: a
 // value keeps up to 62 bits under an exponent shared by the row pair or the test.
 //

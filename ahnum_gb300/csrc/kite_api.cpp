@@ -1,6 +1,6 @@
 // The kite public API (include/kite.h) on top of the GB300 engines: contexts and numbers, the
 // exact host conversions, and the element-wise operations.  Behaviour follows the reference's
-// src/ctx.c:223-559 with the arithmetic backend replaced by kc_* calls (the FP64 IBDWT engine)
+// src/ctx.c:223-559 with the arithmetic backend replaced by kc_* calls (the weighted-transform engine)
 // or kn_* calls (the integer-NTT engine, KITE_BACKEND_CUDA_NTT).
 #include <cstdlib>
 #include <cstring>

@@ -11,7 +11,7 @@
 
 struct kite_ctx {
     kg::Layout lay;            // exact digit layout, weights, N
-    kc_engine *eng = nullptr;  // FP64 IBDWT engine for this modulus, or
+    kc_engine *eng = nullptr;  // weighted-transform engine for this modulus, or
     kn_engine *ntt = nullptr;  // the integer-NTT engine (KITE_BACKEND_CUDA_NTT)
     std::vector<int64_t> dig;  // L digits of host scratch
 };
@@ -22,6 +22,6 @@ struct kite_num {
 
 // x <- x^2 + c, count times, on the context's engine (the LLR doubling with c = -2)
 int kite_square_add_internal(kite_ctx *ctx, kite_num *x, uint64_t count, int64_t c);
-// a == b (mod N): decided on the device by the FP64 engine (kc_equal: 4 bytes read back), by
+// a == b (mod N): decided on the device by the weighted-transform engine (kc_equal: 4 bytes read back), by
 // canonical limbs for the integer-NTT engine.  1 equal, 0 different, negative on a CUDA error.
 int kite_equal_internal(kite_ctx *ctx, const kite_num *a, const kite_num *b);

@@ -36,7 +36,7 @@ bool make_fft_plan(int n, FftPlan &pl);
 std::vector<int4> roots_neg(uint32_t m);
 
 // Shape and column-group width for one test run alone: spread every pass over the SMs so the
-// squaring's latency, not its total FP64 work, is smallest.  Throughput (batched) use takes
+// squaring's latency, not its total work, is smallest (chain_us in plan.cpp).  Throughput (batched) use takes
 // choose_shape and G = kGroup instead.  min_bits: the narrowest digit; top_digits: L - top_t.
 // An autotuned shape of the length (set_latency_override) comes first wherever the number's
 // digits allow its group width.

@@ -153,7 +153,7 @@ def prp(k: int, n: int, base: int = 3, fft_len: int = 0, gerbicz_block: int = 0,
         gerbicz_blocks: int = 0, inject_fault_at: int = 0, checkpoint: str | None = None,
         checkpoint_unverified: str | None = None, checkpoint_secs: float = 0.0,
         unverified_secs: float = 0.0, max_roundoff: float = 0.0, backend: int = CUDA) -> PrpResult:
-    """kite_prp on a CUDA backend (the FP64 engine, or CUDA_NTT)."""
+    """kite_prp on a CUDA backend (the weighted-transform engine, or CUDA_NTT)."""
     lib = native.load()
     o = native.KitePrpOpts()
     o.fft = native.KiteOpts(backend, fft_len, 0, 0)
@@ -188,7 +188,7 @@ class LlrResult:
 def llr(k: int, n: int, fft_len: int = 0, inject_fault_at: int = 0, inject_fault_runs: int = 0,
         inject_roundoff_at: int = 0, inject_roundoff_ladder: int = 0,
         checkpoint: str | None = None, backend: int = CUDA) -> LlrResult:
-    """kite_llr on a CUDA backend (the FP64 engine, or CUDA_NTT)."""
+    """kite_llr on a CUDA backend (the weighted-transform engine, or CUDA_NTT)."""
     lib = native.load()
     o = native.KiteLlrOpts()
     o.fft = native.KiteOpts(backend, fft_len, 0, 0)

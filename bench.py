@@ -19,9 +19,10 @@ advanced by all tests) / (T_blocks * mean(n)).
   e2e       the same through the C ABI with host buffers: wall-clock kc_batch_step calls (their
             H2D slot tables and work lists, D2H round-off), plus per-test admission (H2D of
             x0 and the tables) and read-back (D2H of the residue), amortised per test
-  roofline  a block's algorithmic FP64 FLOPs (its kernels run concurrently on three streams)
-            over the block's CUDA-event time, against the FP64 FMA peak measured on this GPU
-            by a DFMA kernel
+  roofline  a block's algorithmic operations (its kernels run concurrently on three streams) over
+            the block's CUDA-event time, against the least issue time of its 64-bit fixed-point
+            multiplications and additions on the integer pipes; the FP64 pipe's rate, measured by
+            a DFMA kernel, stands beside it
   cpu_baseline  the reference's arithmetic on the host: the CPU oracle's port of the
             reference's `ref` backend (one test per core on all cores) over a bounded sample
 
@@ -215,20 +216,21 @@ PARTS = 3
 # squarings of every test per launch of the persistent kernel, timed beside the block for
 # comparison (the batch's default KITE_GB300_STEPS_PER_LAUNCH)
 STEPS_PER_LAUNCH = 100
-# Per squaring of this workload's 256 tests in the block's form, from one ncu capture of the nine
-# pass launches of one squaring (three parts of three passes; ncu serialises them):
-#   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,sm__sass_thread_inst_executed_op_
-#   {dfma,dadd,dmul}_pred_on.sum,... --clock-control none -k 'regex:k_rows|k_col_inverse|k_col_forward'
-#   -s 256 -c 9 python bench.py --quick --steps 1 --warmup 1 --no-ntt
-# (the 256 launches skipped are the tests' admission).  A block is B + 1 squaring-sized passes.
-# DRAM: 421.9 MB read + 11.2 MB written (ncu runs the three parts one after another; concurrent,
-# the persistent form of the same passes moved 556 MB per squaring).  FP64 lane operations: 479.0e6
-# per squaring on average, from a 100-squaring capture of the same item functions (the single
-# squaring above, 499.9e6, is a step that also tracks round-off, which one step in four does).
-K_SQ_DRAM_BYTES = 433.1e6
-K_SQ_FP64_LANE_OPS = 479.0e6
-K_SQ_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the nine pass launches of one "
-                       "squaring, times B + 1 (profiles/launches_fermat_batch256.md)")
+# DRAM bytes per squaring of this workload's 256 tests, of the row and the column inverse pass: twice an
+# ncu capture of 128 of them (their numbers and tables, 120 MB, already exceed what L2 keeps between
+# passes).
+K_SQ_DRAM_BYTES = 2 * (40.9e6 + 94.3e6)
+K_SQ_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the row and column inverse passes of one "
+                       "squaring of 128 tests, twice, times B + 1 (profiles/fixed_point_passes_batch128.md)")
+
+
+def issue_seconds(lengths: dict, sms: int = 152, clock_hz: float = 2.07e9) -> float:
+    """Least time of one squaring of every test (lengths: FFT length -> tests) on the integer pipes of
+    a GB300 at its maximum clock: per complex point and radix-4 level 57 clocks of issue a warp and
+    quarter SM (three of four inputs times a twiddle at 65, two complex additions at 4), there and
+    back, and 260 for the four-step twiddles, the split, the square and the weights."""
+    points = sum(tests * (L // 2) * (57 * math.log2(L / 2) + 260) for L, tests in lengths.items())
+    return points / 32 / (4 * sms) / clock_hz
 
 
 def run_ours(args):
@@ -335,6 +337,7 @@ def run_ours(args):
     flops_sq = fl3[0] + fl3[1] + fl3[2]          # one squaring of every test
     flops_block = flops_sq * (BLOCK + 1)          # B squarings and the product
     achieved = flops_block / t_block
+    floor_sq = issue_seconds(lengths)
     names = ["k_rows (row FFT + split square), alone", "k_col_inverse (inverse column FFT + round + carry), alone",
              "k_col_forward (carry-in + forward column FFT), alone"]
     kernels = {names[q]: {"ms_per_launch": ms3[q], "gflop_per_launch": fl3[q] / 1e9,
@@ -397,7 +400,7 @@ def run_ours(args):
             "metric": "fermat_tests_per_hour", "value": value, "unit": "tests/hour",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": t_block * 1e3, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded PCG64)",
+            "vs_baseline": None, "dtype": "int64 fixed point", "data": "synthetic (seeded PCG64)",
             "config": bench_config(lengths, mean_n),
             "timed_progress": {"squarings_of_x": progress, "check_blocks": check_blocks,
                                "blocks": args.steps},
@@ -409,20 +412,16 @@ def run_ours(args):
             # per check block two digit passes and the comparison kernel
             "gpu_launches": int(args.steps * (PARTS * 3 * BLOCK + 3) + 3 * check_blocks),
             "clocks": clk.summary(),
-            "roofline": {"bound": "fp64", "achieved": achieved / 1e12, "peak": peak / 1e12,
-                         "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
-                         "traffic": K_SQ_DRAM_BYTES * (BLOCK + 1) if K_SQ_DRAM_BYTES else None,
+            "roofline": {"bound": "integer issue", "achieved": achieved / 1e12,
+                         "peak": flops_sq / floor_sq / 1e12, "unit": "TFLOP/s (algorithmic)",
+                         "frac": floor_sq * (BLOCK + 1) / t_block,
+                         "traffic": K_SQ_DRAM_BYTES * (BLOCK + 1),
                          "traffic_source": K_SQ_TRAFFIC_SOURCE,
-                         # FP64 instructions actually issued (ncu count) against the probe's
-                         # instruction rate (peak / 2: the probe's DFMAs count 2 FLOPs each)
-                         "fp64_issue": None if not K_SQ_FP64_LANE_OPS else {
-                             "lane_ops_per_block": K_SQ_FP64_LANE_OPS * (BLOCK + 1),
-                             "per_second": K_SQ_FP64_LANE_OPS * (BLOCK + 1) / t_block,
-                             "vs_probe_rate": K_SQ_FP64_LANE_OPS * (BLOCK + 1) / t_block / (peak / 2) if peak else None},
+                         "fp64_pipe": {"tflops": peak / 1e12, "block_over_pipe": achieved / peak if peak else None},
                          "kernel": f"one Gerbicz block: the pass kernels of {BLOCK} squarings in {PARTS} parts on "
                                    f"{PARTS} streams, and the product (one CUDA graph; the unit is the block)",
-                         "peak_source": "measured: DFMA dependent-chain kernel on this GPU "
-                                        "(MEASURED_PEAKS.json has no FP64 figure)"},
+                         "peak_source": "the issue clocks of the fixed-point multiplications and additions at "
+                                        "the GPU's maximum SM clock (issue_seconds)"},
             "kernels": kernels,
             "single_test": {"tests_per_hour": single_tph, "us_per_squaring_L49152": us_sq_49152,
                             "us_per_squaring_by_L": {str(L): v * 1e6 for L, v in sorted(single.items())},

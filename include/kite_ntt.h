@@ -1,12 +1,11 @@
 /* Exact integer-NTT squaring engine modulo N = k*2^n - 1 on the GB300 (kn_*).
  *
  * The reference's GPU prototype squares modulo N with an integer number-theoretic transform
- * instead of the FP64 IBDWT (gpu/ntt.metal:121-166, gpu/ntt_reg.metal:90-246, gpu/sq.metal:23-192,
+ * instead of the weighted transform (gpu/ntt.metal:121-166, gpu/ntt_reg.metal:90-246, gpu/sq.metal:23-192,
  * gpu/gpu_ctx.h:57-322): numbers in Montgomery form with R = 2^n, the product P = A + B*2^n
  * (A < 2^n) reduced as P*2^-n == B + k*A (mod N), residues modulo several word-size primes, a
  * Garner CRT back to integers.  This engine restates that arithmetic in CUDA for sm_103a.  It has
- * no round-off at all, so it cross-checks the FP64 engine bit for bit, and it runs on the integer
- * pipes, which GB300 has far more of than FP64 units.
+ * no round-off at all, so it cross-checks the fixed-point engine bit for bit.
  *
  * Representation: a number is W words of w bits (w <= 50) in 64-bit little-endian slots, value
  * x~ = x*2^n mod N up to a small multiple of N.  Three or four primes p < 2^30 with 2^20 | p-1 (per
