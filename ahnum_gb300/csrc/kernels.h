@@ -1,4 +1,4 @@
-// Host-side launch interface of the squaring kernels (kernels.cu).
+// Host-side launch interface of the squaring kernels.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -19,9 +19,9 @@ __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;
 __device__ __forceinline__ void pdl_leave() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // The walk of a pass kernel over its work list.  What does not depend on the previous kernel is done
-// before pdl_enter: the first item's descriptor.  The lists and
-// descriptors are written by copies, which no kernel launched with the attribute overtakes; after a
-// kernel that writes a descriptor the pass is launched without it (LaunchSet::overlap).
+// before pdl_enter: the first item's descriptor.  The lists and descriptors are written by copies,
+// which no kernel launched with the attribute overtakes; after a kernel that writes a descriptor the
+// pass is launched without it (LaunchSet::overlap).
 template <class Item>
 __device__ __forceinline__ void walk_items(const TestDesc *tests, const WorkItem *work, int nwork, int step,
                                            TestDesc *s_desc, ItemCtl *s_ctl, Item &&item) {

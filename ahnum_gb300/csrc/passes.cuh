@@ -1,5 +1,5 @@
 // The passes of a product as device functions over one work item (see device.h for the layout,
-// fixed_fft.cuh for the arithmetic).  The pass kernels (kernels.cu) and the persistent kernel
+// fixed_fft.cuh for the arithmetic).  The pass kernels (rows.cu, columns_*.cu) and the persistent kernel
 // (squarings.cu) run them.
 //
 //   rows_item         row pass: forward row transforms of a row pair, real-split square (or

@@ -216,12 +216,11 @@ PARTS = 3
 # squarings of every test per launch of the persistent kernel, timed beside the block for
 # comparison (the batch's default KITE_GB300_STEPS_PER_LAUNCH)
 STEPS_PER_LAUNCH = 100
-# DRAM bytes per squaring of this workload's 256 tests, of the row and the column inverse pass: twice an
-# ncu capture of 128 of them (their numbers and tables, 120 MB, already exceed what L2 keeps between
-# passes).
-K_SQ_DRAM_BYTES = 2 * (40.9e6 + 94.3e6)
-K_SQ_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the row and column inverse passes of one "
-                       "squaring of 128 tests, twice, times B + 1 (profiles/fixed_point_passes_batch128.md)")
+# DRAM bytes per squaring of this workload's 256 tests: twice an ncu capture of the three passes of
+# 128 of them (their numbers and tables, 120 MB, already exceed what L2 keeps between passes).
+K_SQ_DRAM_BYTES = 2 * (40.9e6 + 94.3e6 + 94.7e6)
+K_SQ_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the three passes of one squaring of 128 "
+                       "tests, twice, times B + 1 (profiles/fixed_point_passes_batch128.md)")
 
 
 def issue_seconds(lengths: dict, sms: int = 152, clock_hz: float = 2.07e9) -> float:
@@ -490,7 +489,7 @@ def ntt_leg(lib, tests, mean_n, device, blocks=3):
     return {"tests_per_hour": tph, "ms_per_block": t_block * 1e3, "ms_per_squaring_step": t_sq * 1e3,
             "us_per_test_squaring": t_sq * 1e6 / len(tests),
             "transform_lengths": {str(k): v for k, v in nps.items()},
-            "gpu_launches_per_squaring": 4,
+            "gpu_launches_per_squaring": 25 / 8,
             "arithmetic": "exact: residues mod three or four 30-bit primes, Garner CRT, Montgomery R=2^n"}
 
 
