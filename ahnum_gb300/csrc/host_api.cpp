@@ -4,6 +4,7 @@
 
 #include "../../include/kite_cuda.h"
 #include "layout.h"
+#include "plan.h"
 
 extern "C" {
 
@@ -43,6 +44,16 @@ int kc_carry_digits(uint64_t k, uint64_t n, uint32_t L, int64_t *digits) {
     if (!y.build(k, n, L)) return -1;
     y.carry(digits);
     return 0;
+}
+
+int kc_transform_plan(int n, int *radix, int *headroom, int *renorm, int *renorm_bits) {
+    kg::FftPlan pl;
+    if (!kg::make_fft_plan(n, pl)) return -1;
+    for (int i = 0; i < pl.ns; i++) radix[i] = pl.stage[i].radix;
+    *headroom = pl.headroom;
+    *renorm = pl.renorm;
+    *renorm_bits = pl.renorm_bits;
+    return pl.ns;
 }
 
 uint32_t kc_choose_fft_len(uint64_t k, uint64_t n) { return kg::choose_fft_len(k, n); }

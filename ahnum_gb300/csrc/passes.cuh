@@ -91,8 +91,9 @@ __device__ __forceinline__ longlong2 as_read(longlong2 v, int, int) { return v; 
 // writes to `to`, the stages then go back and forth between `to` and `alt`, and the last one
 // calls last_st(dst, at, e, l, v, last_pre(e, l)), dst being the buffer it may write to (the value
 // returned) and last_pre what it reads from the tables, asked for before the stage's own work.
-// Long transforms are scaled to their largest component once more on the way (FftPlan::renorm,
-// *mid a zeroed word of the block) by 2^shift, set before the last stage.  Ends with a barrier.
+// Long transforms are scaled up to their largest component once more on the way (FftPlan::renorm,
+// *mid a zeroed word of the block) by 2^shift, shift >= 0, set before the last stage: data that gather on
+// one element have nothing to scale up and are left as they are.  Ends with a barrier.
 template <int LG, bool INV, class TAB, class LD, class COOK, class PRE, class ST>
 __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *tw, longlong2 *to, longlong2 *alt,
                                                 unsigned odd, LD &&first_ld, COOK &&cook, PRE &&last_pre, ST &&last_st, unsigned *mid, int &shift) {
@@ -119,7 +120,7 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
                 });
             if (track) block_or(mag, mid);
             __syncthreads();
-            if (track) shift = 29 - bit_length(*mid);  // components below 2^61
+            if (track) shift = max(0, pl.renorm_bits - 32 - bit_length(*mid));
         } else {
             dispatch_stage<LG, INV, false, false, TAB>(n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; }, as_read, nothing_ahead,
                                                   [&](int at, int, int, longlong2 v, Nothing) { to[at] = v; });

@@ -205,6 +205,7 @@ bool choose_latency_shape(uint32_t H, int nsm, unsigned min_bits, unsigned top_d
 bool make_fft_plan(int n, FftPlan &pl) {
     // The odd radices first (the first stage has span 1 and no twiddles), then a radix 2 if needed,
     // then radix 4; a transform of one stage gets a second one of radix 1.
+    if (n < 2) return false;
     std::vector<int> rad;
     int m = n;
     for (int p : {7, 5, 3})
@@ -215,7 +216,7 @@ bool make_fft_plan(int n, FftPlan &pl) {
         rad.push_back(2);
         m /= 2;
     }
-    if (m != 1 || n < 2) return false;
+    if (m != 1) return false;
     rad.insert(rad.end(), fours, 4);
     if (rad.size() == 1) rad.push_back(1);
     if (rad.size() > (size_t)kMaxStages) return false;
@@ -237,12 +238,25 @@ bool make_fft_plan(int n, FftPlan &pl) {
         s *= p;
         pl.ns++;
     }
-    // half a bit for the modulus of two components
+    // half a bit for the modulus of two components: every modulus then stays below 2^62 in every stage
     pl.headroom = (int)std::ceil(std::log2(largest) + 0.5 - 1e-9);
     // Random data lose half a bit a level against the bound.  Up to four bits of that leave the
     // round-off below half of what FP64 had at the same length; longer transforms take the bits
-    // back before their last two radix-4 stages, else the loss would pass FP64's from 2^9 points on.
-    if (n > 256 && pl.ns >= 3) pl.renorm = pl.ns - 2;
+    // back before their last two stages, else the loss would pass FP64's from 2^9 points on.  Data that
+    // gather on one element keep the bound itself, components up to 2^62, and are never scaled down.
+    // Scaled up to components below 2^61 (moduli below 2^61.5), the last two stages have to stay below
+    // 2^63: their growth is at most 1 where both are of radix 4, 2.5 else, and 3.5 at 686 = 7 7 7 2 alone,
+    // which is scaled to 2^60.  The first stage whose output can be looked at is stage 1.
+    if (n > 256 && pl.ns >= 4) {
+        pl.renorm = pl.ns - 2;
+        double tail = 1, peak = 1;
+        for (int i = pl.renorm; i < pl.ns; i++) {
+            tail *= pl.stage[i].radix > 2 ? pl.stage[i].radix / 4.0 : 2;
+            peak = std::max(peak, tail);
+        }
+        pl.renorm_bits = (int)std::floor(62.9 - 0.5 - std::log2(peak));
+        pl.renorm_bits = std::min(pl.renorm_bits, 61);
+    }
     return true;
 }
 

@@ -1,0 +1,52 @@
+"""The bounds of the fixed-point transforms' plans, for every length that a row or a column can have:
+moduli below 2^62 from the input on, and below 2^63 after the values are scaled up on the way."""
+import ctypes as C
+import math
+from fractions import Fraction
+
+
+def _lengths():
+    def smooth(n):
+        for p in (2, 3, 5, 7):
+            while n % p == 0:
+                n //= p
+        return n == 1
+    return [n for n in range(2, 2049) if smooth(n)]
+
+
+def _growth(i, p):
+    """Bound of a stage's growth of the moduli: twiddled butterflies of radix 3, 4, 5, 7 divide by 4"""
+    return Fraction(p, 4) if i and p > 2 else Fraction(p)
+
+
+def test_plans_of_every_length(lib):
+    scaled = []
+    for n in _lengths():
+        radix, head, renorm, bits = (C.c_int * 8)(), C.c_int(), C.c_int(), C.c_int()
+        ns = lib.kc_transform_plan(n, radix, C.byref(head), C.byref(renorm), C.byref(bits))
+        assert 2 <= ns <= 8 and math.prod(radix[:ns]) == n
+        # squares of moduli: components of 2^b make a modulus of sqrt(2) 2^b
+        at, peak = Fraction(1), Fraction(1)
+        for i in range(ns):
+            at *= _growth(i, radix[i])
+            peak = max(peak, at)
+        assert 2 * (peak * Fraction(2) ** (62 - head.value)) ** 2 <= Fraction(2) ** 124, n
+        if not renorm.value:
+            assert n <= 256 or ns < 4
+            continue
+        scaled.append(n)
+        # stage 1 is the first whose outputs are looked at, and the last stage does not scale
+        assert 2 <= renorm.value <= ns - 2, n
+        assert 32 < bits.value <= 61, n
+        at, peak = Fraction(1), Fraction(1)
+        for i in range(renorm.value, ns):
+            at *= _growth(i, radix[i])
+            peak = max(peak, at)
+        assert 2 * (peak * Fraction(2) ** bits.value) ** 2 < Fraction(2) ** 126 * Fraction(99, 100), n
+    assert {288, 320, 512, 686, 1024, 1440, 2048} <= set(scaled) and 343 not in scaled
+
+
+def test_lengths_without_a_plan(lib):
+    radix, v = (C.c_int * 8)(), [C.c_int() for _ in range(3)]
+    for n in (0, 1, 11, 22, 26, 1331):
+        assert lib.kc_transform_plan(n, radix, *map(C.byref, v)) == -1
