@@ -239,14 +239,12 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
     // a test run alone spreads each pass over the SMs (shape and column-group width chosen for
     // latency); a batch slot takes the throughput shape and the widest groups
     const unsigned top_digits = e->lay.L - e->lay.top_t;
+    unsigned min_bits = 64;
+    for (uint8_t b : e->lay.bits) min_bits = b < min_bits ? b : min_bits;
     if (throughput) {
-        e->G = kGroup;
-        e->plan = get_plan(L);
-        // a column group's two buffers have to fit shared memory
-        if (e->plan && 2 * (size_t)e->plan->R * e->G * sizeof(longlong2) > kMaxColSmem) e->G = 4;
+        uint32_t R = 0;
+        if (throughput_group(L / 2, min_bits, top_digits, R, e->G)) e->plan = get_plan(L, R);
     } else {
-        unsigned min_bits = 64;
-        for (uint8_t b : e->lay.bits) min_bits = b < min_bits ? b : min_bits;
         int nsm = 1;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
         uint32_t R = 0, C = 0;

@@ -43,6 +43,9 @@ static bool shape_usable(uint32_t H, uint32_t r, uint32_t c) {
            factorable(r) && factorable(c);
 }
 
+// a column group's two buffers fit shared memory: up to 896 rows in groups of 8, always in narrower ones
+static bool column_fits(uint32_t r, int g) { return 2 * (size_t)r * g * sizeof(int4) <= kMaxColSmem; }
+
 // Shapes chosen by the autotuner (or a tuning file), by FFT length L = 2H: R rows.
 static std::mutex g_shape_mu;
 static std::map<uint32_t, uint32_t> g_shape;
@@ -155,6 +158,22 @@ static bool group_fits(int g, unsigned min_bits, unsigned top_digits) {
     return (2 * g - 1) * (int)min_bits >= 51 - (int)min_bits && (int)top_digits <= 2 * g;
 }
 
+bool throughput_group(uint32_t H, unsigned min_bits, unsigned top_digits, uint32_t &R, int &G) {
+    uint32_t C = 0;
+    if (!choose_shape(H, R, C)) return false;
+    G = kGroup;
+    if (column_fits(R, G)) return (int)top_digits <= 2 * G;
+    G = kGroup / 2;
+    if (group_fits(G, min_bits, top_digits)) return true;
+    for (uint32_t c = 16; c <= 2048 && c <= H / 2; c += kGroup)
+        if (H % c == 0 && shape_usable(H, H / c, c) && column_fits(H / c, kGroup)) {
+            R = H / c;  // the longest columns that fit groups of 8
+            G = kGroup;
+            break;
+        }
+    return (int)top_digits <= 2 * G;
+}
+
 bool set_latency_override(uint32_t L, uint32_t R, int G) {
     std::lock_guard<std::mutex> lock(g_shape_mu);
     if (!R) {
@@ -174,10 +193,11 @@ bool choose_latency_shape(uint32_t H, int nsm, unsigned min_bits, unsigned top_d
         // an autotuned shape of this length, where this number's digits allow its groups
         std::lock_guard<std::mutex> lock(g_shape_mu);
         auto it = g_latency.find(2 * H);
-        if (it != g_latency.end() && group_fits(it->second.second, min_bits, top_digits)) {
+        const int g = it == g_latency.end() ? 0 : column_fits(it->second.first, it->second.second) ? it->second.second : kGroup / 2;
+        if (g && group_fits(g, min_bits, top_digits)) {
             R = it->second.first;
             C = H / R;
-            G = it->second.second;
+            G = g;
             return true;
         }
     }
@@ -185,21 +205,29 @@ bool choose_latency_shape(uint32_t H, int nsm, unsigned min_bits, unsigned top_d
     R = C = 0;
     G = kGroup;
     if (nsm < 1) nsm = 1;
-    for (uint32_t c = 16; c <= 2048 && c <= H / 2; c += kGroup) {
-        if (H % c || !shape_usable(H, H / c, c)) continue;
-        const uint32_t r = H / c;
-        for (int g : {2, 4, 8}) {
-            if (!group_fits(g, min_bits, top_digits)) continue;
-            const double cost = chain_us(r, c, g, nsm) + (r < 4 ? 1e3 : 0);  // two rows: where nothing else fits
-            if (cost < best - 1e-9) {
-                best = cost;
-                R = r;
-                C = c;
-                G = g;
+    // The second round: where columns are too long for groups of 8 at every shape (from L = 3670017 on),
+    // digits that ask for 8 take groups of 4 all the same; the last digit of a segment keeps what the
+    // others leave of a carry (TestDesc::digit_bits).
+    const bool fits8 = group_fits(kGroup, min_bits, top_digits);
+    for (bool narrow : {false, true}) {
+        for (uint32_t c = 16; c <= 2048 && c <= H / 2; c += kGroup) {
+            if (H % c || !shape_usable(H, H / c, c)) continue;
+            const uint32_t r = H / c;
+            for (int g : {2, 4, 8}) {
+                if (!column_fits(r, g)) continue;
+                if (!group_fits(g, min_bits, top_digits) && !(narrow && fits8 && g == 4 && (int)top_digits <= 2 * g)) continue;
+                const double cost = chain_us(r, c, g, nsm) + (r < 4 ? 1e3 : 0);  // two rows: where nothing else fits
+                if (cost < best - 1e-9) {
+                    best = cost;
+                    R = r;
+                    C = c;
+                    G = g;
+                }
             }
         }
+        if (R) return true;
     }
-    return R != 0;
+    return false;
 }
 
 bool make_fft_plan(int n, FftPlan &pl) {

@@ -25,6 +25,10 @@ struct LengthPlan {
 // H = R*C with C a multiple of kGroup; the autotuned shape of this length if one was set, else
 // rows about four times as long as columns.  false if no usable shape exists.
 bool choose_shape(uint32_t H, uint32_t &R, uint32_t &C);
+// Rows and column-group width of a batch slot: choose_shape's rows and groups of 8.  Columns of more than
+// 896 rows leave no room for 8: groups of 4, or, where the number's digits ask for 8 (min_bits: the
+// narrowest; top_digits: L - top_t), the longest columns that do.  false if no shape takes the number.
+bool throughput_group(uint32_t H, unsigned min_bits, unsigned top_digits, uint32_t &R, int &G);
 // Use R rows for FFT length L from now on (R = 0: back to the default); false if unusable.
 bool set_shape_override(uint32_t L, uint32_t R);
 // Usable shapes of H = R*C near balance, at most `max`; returns the count.

@@ -79,7 +79,7 @@ void *kc_stream(kc_engine *e);
 /* Four-step shape chosen for the engine's length: H = R * C complex points. */
 void kc_shape(const kc_engine *e, uint32_t *R, uint32_t *C);
 /* Columns per column-pass work unit (2, 4 or 8): an engine created by kc_engine_new spreads each
- * pass of one squaring over the SMs; batch slots use 8. */
+ * pass of one squaring over the SMs; batch slots use 8, or 4 with more than 896 rows. */
 int kc_group_width(const kc_engine *e);
 /* Self-test of the bounded waits between CTAs (no counterpart in the reference, whose host threads
  * never wait on one another on a device).  Launches the batch's persistent kernel over engine e's
@@ -230,7 +230,8 @@ int kc_fft_shape_candidates(uint32_t L, uint32_t *R, uint32_t *C, int max);
 int kc_fft_shape(uint32_t L, uint32_t *R, uint32_t *C);
 /* Shape of one test run alone (latency mode, kc_engine_new with throughput 0) at length L:
  * R rows and column groups of G in {2, 4, 8} (R = 0: back to the built-in model).  Used for
- * every number whose digits allow groups of G.  0, or -1 if the shape is unusable. */
+ * every number whose digits allow groups of G; more than 896 rows take groups of 4 where G is 8.
+ * 0, or -1 if the shape is unusable. */
 int kc_set_latency_shape(uint32_t L, uint32_t R, int G);
 /* Load a tuning file (shapes and times).  Lines "L us R C G" (five fields) are latency shapes
  * (kc_set_latency_shape; their times, single-test microseconds, do not steer the length
