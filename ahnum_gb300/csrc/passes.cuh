@@ -440,6 +440,9 @@ __device__ __forceinline__ long long scale_round(long long v, long long u, int n
     return q - (frac >> 31);
 }
 
+// |frac| times 2^32: a half, which is the lowest int, too
+__device__ __forceinline__ unsigned distance(int frac) { return frac < 0 ? 0u - (unsigned)frac : (unsigned)frac; }
+
 // The scale of a column inverse whose components are below 2^e: conj(t4) divides by 4
 __device__ __forceinline__ int col_scale(const FftPlan &pl, int e) {
     return 64 - max(3, pl.headroom) - e;
@@ -529,7 +532,7 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
             int fx, fy;
             v.x = scale_round(v.x, o.x, m, fx);
             v.y = scale_round(v.y, o.y, m, fy);
-            err = max(err, (unsigned)max(abs(fx), abs(fy)));
+            err = max(err, max(distance(fx), distance(fy)));
             big |= mag32(v);
             dst[turned<LG>(r, l)] = v;
         },
