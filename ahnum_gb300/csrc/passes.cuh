@@ -440,9 +440,6 @@ __device__ __forceinline__ long long scale_round(long long v, long long u, int n
     return q - (frac >> 31);
 }
 
-// |frac| times 2^32: a half, which is the lowest int, too
-__device__ __forceinline__ unsigned distance(int frac) { return frac < 0 ? 0u - (unsigned)frac : (unsigned)frac; }
-
 // The scale of a column inverse whose components are below 2^e: conj(t4) divides by 4
 __device__ __forceinline__ int col_scale(const FftPlan &pl, int e) {
     return 64 - max(3, pl.headroom) - e;
@@ -518,7 +515,8 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
     const unsigned odd = odd_columns(g, LG);
     int shift;
     const long long *osc = T.osc + 2 * (g << LG);
-    unsigned err = 0, big = 0;
+    int above = 0, below = 0;  // the largest difference to an integer of either sign
+    unsigned big = 0;
     longlong2 *digits = transform<LG, true, TAB>(
         pl, T.twc, sm, sm + (T.R << LG), odd,
         [&](int, int k, int l) { return TurnedIn{__ldcg(&x[k * C + l]), TAB::load(&t4[k * T.pitch + l]), __ldcg(&rexp[k])}; },
@@ -532,7 +530,8 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
             int fx, fy;
             v.x = scale_round(v.x, o.x, m, fx);
             v.y = scale_round(v.y, o.y, m, fy);
-            err = max(err, max(distance(fx), distance(fy)));
+            above = max(above, max(fx, fy));
+            below = min(below, min(fx, fy));
             big |= mag32(v);
             dst[turned<LG>(r, l)] = v;
         },
@@ -540,7 +539,8 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
     const bool short_transform = n + shift < 0;  // the last place is above 1: too short for its data
     segment_carries<1 << LG, TAB>(T, g, digits);
     // |digit| >= 2^51 reports 0.5, as does a transform too short for its data
-    if (!track) err = 0;
+    // below in unsigned: -1/2 is the lowest int
+    unsigned err = track ? max((unsigned)above, 0u - (unsigned)below) : 0;
     if (big >= (1u << 19) || short_transform) err = 0x80000000u;
     err = __reduce_max_sync(0xffffffffu, err);
     if ((threadIdx.x & 31) == 0 && err)
