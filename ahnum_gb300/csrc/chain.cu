@@ -23,39 +23,54 @@ static bool keeps_tables(const LaunchSet &s, int nsm) {
 }
 size_t chain_smem(const LaunchSet &s, int nsm) { return work_smem(s) + (keeps_tables(s, nsm) ? s.table_smem : 0); }
 
-bool chain_in_cluster(const LaunchSet &s) { return std::max(s.nrows, s.ncols) <= kClusterItems; }
-
-int chain_grid(const LaunchSet &s, int nsm) {
-    if (chain_in_cluster(s)) {
-        int grid = 1;
-        while (grid < std::max(s.nrows, s.ncols)) grid *= 2;
-        return grid;
-    }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, by_group(s.G, k_chain<1, false>, k_chain<2, false>, k_chain<3, false>),
-                                                      kThreads, chain_smem(s, nsm)) != cudaSuccess)
-        return 0;
-    return std::min(per_sm * nsm, std::max(s.nrows, s.ncols));
+static int cluster_size(const LaunchSet &s) {
+    int size = 1;
+    while (size < std::max(s.nrows, s.ncols)) size *= 2;
+    return size;
 }
 
-cudaError_t launch_chain(const LaunchSet &s, int nsm, int grid, bool cluster, double2 *x, int step0, int nsteps, ChainCtl *ctl,
-                         unsigned arrived, unsigned *flags, unsigned done, long long limit) {
+static cudaLaunchConfig_t chain_config(const LaunchSet &s, int nsm, int grid, bool cluster, cudaLaunchAttribute *at) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = chain_smem(s, nsm);
     cfg.stream = s.stream;
-    cudaLaunchAttribute at[1];
     if (cluster) {
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = grid;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = grid;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
     } else {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
+        at->id = cudaLaunchAttributeCooperative;
+        at->val.cooperative = 1;
     }
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    return cfg;
+}
+
+bool chain_in_cluster(const LaunchSet &s) { return std::max(s.nrows, s.ncols) <= kClusterItems; }
+
+int chain_grid(const LaunchSet &s, int nsm, bool cluster) {
+    if (cluster) return cluster_size(s);
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, by_group(s.G, k_chain<1, false>, k_chain<2, false>, k_chain<3, false>),
+                                                      kThreads, chain_smem(s, nsm)) != cudaSuccess)
+        return 0;
+    // as many as there are items, or the fewest that take them in the same number of rounds: the
+    // places that are left serve other contexts' kernels
+    const int most = std::min(per_sm * nsm, std::max(s.nrows, s.ncols));
+    if (most < 1) return 0;
+    const auto fewest = [&](int items) {
+        const int rounds = (items + most - 1) / most;
+        return (items + rounds - 1) / rounds;
+    };
+    return std::max(fewest(s.nrows), fewest(s.ncols));
+}
+
+cudaError_t launch_chain(const LaunchSet &s, int nsm, int grid, bool cluster, double2 *x, int step0, int nsteps, ChainCtl *ctl,
+                         unsigned arrived, unsigned *flags, unsigned done, long long limit) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = chain_config(s, nsm, grid, cluster, &at);
     const ChainKernel k = cluster ? chain_cluster_kernel(s.G) : by_group(s.G, k_chain<1, false>, k_chain<2, false>, k_chain<3, false>);
     return cudaLaunchKernelEx(&cfg, k, s.tests, x, step0, nsteps,
                               keeps_tables(s, nsm) ? (int)(work_smem(s) / sizeof(longlong2)) : 0, ctl, arrived, flags, done, limit);

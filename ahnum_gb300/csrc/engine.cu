@@ -79,6 +79,9 @@ bool dalloc(kc_engine *e, T **p, size_t count) {
 }
 
 void release(kc_engine *e) {
+    if (e->graph) cudaGraphExecDestroy(e->graph);
+    for (cudaEvent_t m : e->marks)
+        if (m) cudaEventDestroy(m);
     cudaFree(e->d_desc);
     cudaFree(e->d_work);
     cudaFree(e->d_bits);
@@ -138,39 +141,128 @@ int product(kc_engine *e, double2 *x, const double2 *y) {
     return check_launch(e) ? 0 : e->err;
 }
 
-// Cooperative chains wait on their own CTAs, so two of them must not be on the device at once: each one
-// is put behind the previous one of the device, whichever engine launched it.  A cluster's CTAs start
-// together and need none of this.
-struct ChainQueue {
-    std::mutex mu;
-    cudaEvent_t last = nullptr;
-    cudaStream_t stream = nullptr;  // of the last chain
+// Calls between a caller's kernels that a capture in another thread must not forbid or be ended by
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
-ChainQueue g_chains[kMaxDevices];
 
-// count squarings of x
-int square_many(kc_engine *e, double2 *x, uint64_t count) {
-    ChainQueue &q = g_chains[e->device];
-    while (count) {
-        const int n = (int)std::min(count, kChainSteps);
-        if (e->chain_cluster) {
-            if (!ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, true, x, (int)(e->op_count % e->err_every), n, e->d_chain, 0, nullptr, 0)))
-                return e->err;
-            e->op_count += (uint64_t)n;
-            count -= (uint64_t)n;
+bool capturing(const kc_engine *e) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(e->stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
+// The engines of a device that squared alone and may still have work in their queues
+struct Device {
+    std::mutex mu;
+    std::vector<kc_engine *> busy;
+};
+Device g_devices[kMaxDevices];
+
+// Whether e's next squarings, which it launches under dev.mu, can be a chain.
+//
+// A chain's CTAs wait on one another, so all of them have to become resident, and they stay for
+// milliseconds.  Chains whose CTAs together have an SM each run side by side; where the engines with
+// work queued leave no room for that, the squarings run as launches of the pass kernels, which wait on
+// nothing and share the SMs.  us per squaring of all contexts together on GB300, one thread each, with
+// chains behind one another -> by this rule, for 1, 2, 4 and 8 contexts of the same length:
+//   3584 digits    13.9 13.9 13.7 13.6 -> 14.2  7.1  3.5  2.6   49152   17.6 17.5 17.5 17.5 -> 17.5 11.9  6.4  4.2
+//   28672          17.0 16.9 16.9 16.9 -> 16.0  8.2  5.6  3.5   442368  34.2 34.2 34.3 34.4 -> 34.5 33.1 22.8 17.7
+bool chain_has_room(Device &dev, const kc_engine *e) {
+    const RelaxedCapture relaxed;
+    int others = 0;
+    for (size_t i = 0; i < dev.busy.size();) {
+        const kc_engine *o = dev.busy[i];
+        if (o != e && !capturing(o) && cudaStreamQuery(o->stream) != cudaErrorNotReady) {
+            dev.busy[i] = dev.busy.back();
+            dev.busy.pop_back();
             continue;
         }
-        std::lock_guard<std::mutex> lock(q.mu);
-        if (!q.last && !ok(e, cudaEventCreateWithFlags(&q.last, cudaEventDisableTiming))) return e->err;
-        if (q.stream != e->stream && !ok(e, cudaStreamWaitEvent(e->stream, q.last, 0))) return e->err;
-        if (!ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, false, x, (int)(e->op_count % e->err_every), n, e->d_chain, e->arrived,
-                                e->d_flags, e->chained)) ||
-            !ok(e, cudaEventRecord(q.last, e->stream)))
-            return e->err;
-        q.stream = e->stream;
-        e->arrived += 2u * (unsigned)n * (unsigned)e->chain_grid;
-        e->chained += (unsigned)n;
-        e->op_count += (uint64_t)n;
+        if (o != e) others += o->chain_grid;
+        i++;
+    }
+    if (others) (void)cudaGetLastError();  // not ready is no error
+    return !others || others + e->chain_grid <= e->nsm;
+}
+
+// A graph of kGraphSteps squarings by the pass kernels, of the number in the second descriptor
+bool make_graph(kc_engine *e) {
+    if (e->graph) return true;
+    const RelaxedCapture relaxed;
+    LaunchSet s = e->ls;
+    s.tests = e->d_desc + 1;
+    cudaGraph_t graph = nullptr;
+    if (!ok(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed))) return false;
+    for (int j = 0; j < (int)kGraphSteps; j++) {
+        launch_rows(s, false, nullptr, nullptr, j);
+        launch_col_inverse(s, nullptr, j);
+        launch_col_forward(s, nullptr, true, j);
+    }
+    if (!ok(e, cudaStreamEndCapture(e->stream, &graph))) return false;
+    const bool made = ok(e, cudaGraphInstantiate(&e->graph, graph, 0));
+    cudaGraphDestroy(graph);
+    return made;
+}
+
+// n squarings of x as launches of the pass kernels: graphs, and the rest one by one
+int square_passes(kc_engine *e, double2 *x, uint64_t n) {
+    for (; n >= kGraphSteps; n -= kGraphSteps) {
+        if (!make_graph(e)) return e->err ? e->err : -1;
+        TestDesc d = e->desc;
+        d.x = x;
+        if (std::memcmp(&d, &e->graph_desc, sizeof d)) {
+            std::memcpy(&e->graph_desc, &d, sizeof d);
+            if (!ok(e, cudaMemcpyAsync(e->d_desc + 1, &e->graph_desc, sizeof d, cudaMemcpyHostToDevice, e->stream))) return e->err;
+        }
+        if (!ok(e, cudaGraphLaunch(e->graph, e->stream))) return e->err;
+        e->op_count += kGraphSteps;
+    }
+    for (; n; n--)
+        if (product(e, x, nullptr)) return e->err;
+    return 0;
+}
+
+// The form of the squarings follows what other engines do, so the queue does not run far ahead of the
+// GPU: waits until fewer than 3 kAhead squarings of this engine are queued, n of them new.
+bool limit_ahead(kc_engine *e, uint64_t n) {
+    e->ahead += n;
+    if (e->ahead < kAhead) return true;
+    const RelaxedCapture relaxed;
+    e->ahead = 0;
+    cudaEvent_t &mark = e->marks[e->turn ^= 1];
+    if (mark ? !ok(e, cudaEventSynchronize(mark)) : !ok(e, cudaEventCreateWithFlags(&mark, cudaEventBlockingSync | cudaEventDisableTiming)))
+        return false;
+    return ok(e, cudaEventRecord(mark, e->stream));
+}
+
+// count squarings of x.  A batch slot's few go by the pass kernels.
+int square_many(kc_engine *e, double2 *x, uint64_t count) {
+    if (e->throughput) {
+        for (; count; count--)
+            if (product(e, x, nullptr)) return e->err;
+        return 0;
+    }
+    Device &dev = g_devices[e->device];
+    while (count) {
+        const int n = (int)std::min(count, e->chain_steps);
+        if (!limit_ahead(e, (uint64_t)n)) return e->err;
+        std::unique_lock<std::mutex> lock(dev.mu);
+        const bool chain = e->chain_cluster || chain_has_room(dev, e);
+        if (std::find(dev.busy.begin(), dev.busy.end(), e) == dev.busy.end()) dev.busy.push_back(e);
+        if (e->chain_cluster || !chain) lock.unlock();  // nothing that has to fit beside another chain
+        if (!chain) {
+            if (square_passes(e, x, (uint64_t)n)) return e->err;
+        } else {
+            if (!ok(e, launch_chain(e->ls, e->nsm, e->chain_grid, e->chain_cluster, x, (int)(e->op_count % e->err_every), n, e->d_chain,
+                                    e->arrived, e->d_flags, e->chained)))
+                return e->err;
+            if (!e->chain_cluster) {
+                e->arrived += 2u * (unsigned)n * (unsigned)e->chain_grid;
+                e->chained += (unsigned)n;
+            }
+            e->op_count += (uint64_t)n;
+        }
         count -= (uint64_t)n;
     }
     return 0;
@@ -224,6 +316,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         return nullptr;
     }
     e->device = device;
+    e->throughput = throughput;
     DeviceGuard dg(device);
     if (!e->lay.build(k, n, L)) {
         delete e;
@@ -264,7 +357,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
     // the chain's words after the exponents and emax, aligned; its flags after those
     const size_t chain_at = ((size_t)P.R + 3) & ~(size_t)1, flags_at = (chain_at + sizeof(ChainCtl) / sizeof(int) + 7) & ~(size_t)7;
     bool good = ok(e, cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) &&
-                dalloc(e, &e->d_desc, 1) && dalloc(e, &e->d_work, P.pairs.size() + e->NG) &&
+                dalloc(e, &e->d_desc, 2) && dalloc(e, &e->d_work, P.pairs.size() + e->NG) &&
                 dalloc(e, &e->d_bits, 2 * (size_t)L) && dalloc(e, &e->d_w, L) && dalloc(e, &e->d_osc, L) &&
                 dalloc(e, &e->d_idig, L) && dalloc(e, &e->d_dig, L) && dalloc(e, &e->d_dig2, L) &&
                 dalloc(e, &e->d_eq, 1) && ok(e, cudaMallocHost((void **)&e->h_eq, sizeof(int))) &&
@@ -366,8 +459,9 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         s.table_smem = ((size_t)2 * P.C + P.R + 4 * (size_t)P.R * e->G) * 16 + ((size_t)2 * P.R * e->G + 15) / 16 * 16;
         good = good && ok(e, cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device)) &&
                kernels_prepare(s.row_smem_per_lane * 6, s.col_smem, chain_smem(s, e->nsm)) == 0;
-        e->chain_cluster = chain_in_cluster(s);
-        e->chain_grid = good ? chain_grid(s, e->nsm) : 0;
+        e->chain_cluster = good && chain_in_cluster(s);
+        e->chain_grid = good ? chain_grid(s, e->nsm, e->chain_cluster) : 0;
+        e->chain_steps = std::max<uint64_t>(32, std::min<uint64_t>(512, kChainDigits / L));
         good = e->chain_grid > 0;
     }
     if (!good) {
@@ -395,6 +489,11 @@ void kc_engine_free(kc_engine *e) {
     if (!e) return;
     DeviceGuard dg(e->device);
     cudaStreamSynchronize(e->stream);
+    {
+        Device &dev = g_devices[e->device];
+        std::lock_guard<std::mutex> lock(dev.mu);
+        dev.busy.erase(std::remove(dev.busy.begin(), dev.busy.end(), e), dev.busy.end());
+    }
     release(e);
     delete e;
 }
@@ -511,7 +610,7 @@ void kc_set_roundoff_check(kc_engine *e, uint32_t every) {
     e->err_every = every ? every : 1;
     if (e->desc.err_every != (int)e->err_every) {
         DeviceGuard dg(e->device);
-        e->desc.err_every = (int)e->err_every;  // read by the graphed squarings
+        e->desc.err_every = (int)e->err_every;  // read by chains and graphs
         upload_desc(e);
     }
 }

@@ -43,9 +43,24 @@ struct kc_engine {
     unsigned chained = 0;
     bool chain_cluster = false;
     int chain_grid = 0, nsm = 0;
+    uint64_t chain_steps = 0;          //   squarings per launch, at most
+    bool throughput = false;           // a batch slot's: squares by the pass kernels
+    // squarings by the pass kernels where a chain has no room, kGraphSteps a graph of the number that the
+    // second descriptor at d_desc names, graph_desc being its copy
+    cudaGraphExec_t graph = nullptr;
+    kg::TestDesc graph_desc{};
+    cudaEvent_t marks[2] = {};         // after each kAhead squarings queued, in turn
+    int turn = 0;
+    uint64_t ahead = 0;                // squarings since the last mark
 };
 
-constexpr uint64_t kChainSteps = 512;  // squarings per launch: some 5 ms, 60 ms at the longest lengths
+// Squarings of a chain's launch: up to 512 (7 ms at 28672 digits) and 2^26 digits in all (4 ms at 1769472),
+// since a chain that takes all SMs keeps other contexts' kernels waiting that long.  us per squaring with
+// 32, 128 and 512 a launch: 14.2, 14.1, 14.0 at 3584 digits, 21.4, 21.2, 20.9 at 163840, 98.4, 98.2, 97.9 at
+// 1769472.
+constexpr uint64_t kChainDigits = 1ull << 26;
+constexpr uint64_t kGraphSteps = 16;
+constexpr uint64_t kAhead = 8192;  // 140 ms at 28672 digits
 
 // kc_engine_new for a test run alone (throughput = false: shape and group width chosen for the
 // latency of one squaring) or for a batch slot (throughput = true: the throughput shape, G = 8).

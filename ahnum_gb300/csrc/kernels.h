@@ -102,7 +102,7 @@ cudaError_t launch_chain(const LaunchSet &s, int nsm, int grid, bool cluster, do
 bool chain_in_cluster(const LaunchSet &s);
 // CTAs of a chain: one per item of the larger pass (a power of two in a cluster), at most what is
 // resident at once; 0 on failure.
-int chain_grid(const LaunchSet &s, int nsm);
+int chain_grid(const LaunchSet &s, int nsm, bool cluster);
 size_t chain_smem(const LaunchSet &s, int nsm);  // its dynamic shared memory
 int chain_set_smem(size_t bytes);
 // op: 0 copy, 1 add, 2 sub

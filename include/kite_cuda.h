@@ -46,7 +46,8 @@ int kc_from_digits(kc_engine *e, double *x, const int64_t *digits);
 int kc_to_digits(kc_engine *e, const double *x, int64_t *digits);
 
 /* Replace kite_backend_ops.square / mul (src/internal.h:64-65) and the loop of kite_square_n
- * (src/ctx.c:329-331).  Queued on the engine's stream; return without waiting. */
+ * (src/ctx.c:329-331).  Queued on the engine's stream; return without waiting, but for a kc_square or
+ * kc_square_add that would leave more than about 24000 squarings queued: it waits for some of them. */
 int kc_square(kc_engine *e, double *x, uint64_t count);
 int kc_mul(kc_engine *e, double *x, const double *y);
 /* x <- x^2 + c (c a small signed constant in value terms, e.g. -2 for the LLR step
