@@ -236,9 +236,10 @@ bool limit_ahead(kc_engine *e, uint64_t n) {
     return ok(e, cudaEventRecord(mark, e->stream));
 }
 
-// count squarings of x.  A batch slot's few go by the pass kernels.
+// count squarings of x.  A batch slot's few go by the pass kernels, and so do those that a caller
+// captures: a chain counts its meetings from launch to launch and cannot be replayed.
 int square_many(kc_engine *e, double2 *x, uint64_t count) {
-    if (e->throughput) {
+    if (e->throughput || capturing(e)) {
         for (; count; count--)
             if (product(e, x, nullptr)) return e->err;
         return 0;

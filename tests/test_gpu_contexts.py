@@ -1,5 +1,6 @@
 """Several contexts with work at once: their squarings share the GPU instead of running one after another,
-and are right in either form, whatever the count, the addend and how often the round-off is tracked."""
+and are right in either form, whatever the count, the addend and how often the round-off is tracked; and
+squarings that a caller captures on the engine's stream can be replayed."""
 import ctypes as C
 import random
 import threading
@@ -91,3 +92,35 @@ def test_squares_beside_another(lib, L):
             lib.kc_num_free(e, x)
             lib.kc_engine_free(e)
     assert ends[0] == ends[2] and ends[1] == ends[3]
+
+
+@pytest.mark.parametrize("L", [1344, 3584])
+def test_captured_squarings_replay(lib, L):
+    torch = pytest.importorskip("torch")
+    n = 11 * L
+    e = lib.kc_engine_new(K, n, L, None, None, None, 0, 0, 0, 0, -1)
+    assert e
+    x = lib.kc_num_alloc(e)
+    try:
+        digits = (C.c_int64 * L)(3)
+        assert lib.kc_from_digits(e, x, digits) == 0
+        assert lib.kc_square(e, x, 40) == 0 and lib.kc_sync(e) == 0
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(torch.cuda.ExternalStream(lib.kc_stream(e))):
+            graph.capture_begin(capture_error_mode="thread_local")
+            assert lib.kc_square(e, x, 5) == 0
+            graph.capture_end()
+            for _ in range(4):
+                graph.replay()
+        assert lib.kc_square(e, x, 20) == 0
+        assert lib.kc_to_digits(e, x, digits) == 0
+        limbs = (C.c_uint64 * ((n + 127) // 64))()
+        assert lib.kc_digits_to_limbs(K, n, L, digits, limbs) == 0
+        v = 3 * K
+        for _ in range(80):
+            v = _mod(v * v, K, n)
+        assert int.from_bytes(bytes(limbs), "little") == v
+        assert lib.kc_error(e) == 0
+    finally:
+        lib.kc_num_free(e, x)
+        lib.kc_engine_free(e)
