@@ -48,7 +48,16 @@ static cudaLaunchConfig_t chain_config(const LaunchSet &s, int nsm, int grid, bo
     return cfg;
 }
 
-bool chain_in_cluster(const LaunchSet &s) { return std::max(s.nrows, s.ncols) <= kClusterItems; }
+bool chain_in_cluster(const LaunchSet &s, int nsm) {
+    if (std::max(s.nrows, s.ncols) > kClusterItems) return false;
+    // a part of a GPU may have no place for that many CTAs side by side: then cooperatively
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = chain_config(s, nsm, cluster_size(s), true, &at);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, chain_cluster_kernel(s.G), &cfg) == cudaSuccess && clusters > 0) return true;
+    (void)cudaGetLastError();
+    return false;
+}
 
 int chain_grid(const LaunchSet &s, int nsm, bool cluster) {
     if (cluster) return cluster_size(s);

@@ -460,7 +460,7 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         s.table_smem = ((size_t)2 * P.C + P.R + 4 * (size_t)P.R * e->G) * 16 + ((size_t)2 * P.R * e->G + 15) / 16 * 16;
         good = good && ok(e, cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device)) &&
                kernels_prepare(s.row_smem_per_lane * 6, s.col_smem, chain_smem(s, e->nsm)) == 0;
-        e->chain_cluster = good && chain_in_cluster(s);
+        e->chain_cluster = good && chain_in_cluster(s, e->nsm);
         e->chain_grid = good ? chain_grid(s, e->nsm, e->chain_cluster) : 0;
         e->chain_steps = std::max<uint64_t>(32, std::min<uint64_t>(512, kChainDigits / L));
         good = e->chain_grid > 0;

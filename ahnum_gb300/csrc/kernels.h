@@ -99,7 +99,7 @@ constexpr int kFlagWords = 8;      // one 32-byte sector
 constexpr int kClusterItems = 16;  // the largest cluster
 cudaError_t launch_chain(const LaunchSet &s, int nsm, int grid, bool cluster, double2 *x, int step0, int nsteps, ChainCtl *ctl,
                          unsigned arrived, unsigned *flags, unsigned done, long long limit = kWaitCycles);
-bool chain_in_cluster(const LaunchSet &s);
+bool chain_in_cluster(const LaunchSet &s, int nsm);
 // CTAs of a chain: one per item of the larger pass (a power of two in a cluster), at most what is
 // resident at once; 0 on failure.
 int chain_grid(const LaunchSet &s, int nsm, bool cluster);
