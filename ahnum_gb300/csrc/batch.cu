@@ -729,7 +729,7 @@ int kc_batch_step(kc_batch *b, uint32_t blocks, double *gpu_ms) {
         if (sq.empty()) break;
         size_t row_lane, col_smem;
         max_smem(b, row_lane, col_smem);
-        int form = b->persistent && !has_narrow(b) ? kPersistent : kPerPass;
+        int form = b->persistent ? kPersistent : kPerPass;
         const int nparts = form == kPerPass ? std::min<int>(b->parts, (int)sq.size()) : 1;
         if (nparts >= 2) form = kSplit;
         // the lists: all slots in part 0, or a split block's parts of about equal work (row pairs
@@ -1052,7 +1052,7 @@ int kc_batch_profile_steps(kc_batch *b, uint32_t squarings, double *ms, double *
         const double H = P.H, L = P.L;
         fl += 10.0 * H * std::log2((double)P.C) + 10.0 * L + 2 * (5.0 * H * std::log2((double)P.R) + 7.0 * L);
     }
-    if (sq.empty() || has_narrow(b)) return -1;
+    if (sq.empty()) return -1;
     size_t row_lane, col_smem;
     max_smem(b, row_lane, col_smem);
     row_lane = std::max(row_lane, b->graph_row_smem);
