@@ -34,7 +34,7 @@ struct ItemCtl {
     unsigned mag[2];    //   OR of the upper words of |component| after the forward transform
     unsigned mag_split; //   after the split
     unsigned mag_out;   //   after the inverse transform
-    unsigned mid[3][2]; //   before FftPlan::renorm and early: the transforms of x and y, and the inverse
+    unsigned mid[3];    //   before FftPlan::renorm: the transforms of x and y, and the inverse
 };
 
 // The work item's test descriptor, copied into shared memory.  An item reads the descriptor's
@@ -91,14 +91,13 @@ __device__ __forceinline__ longlong2 as_read(longlong2 v, int, int) { return v; 
 // writes to `to`, the stages then go back and forth between `to` and `alt`, and the last one
 // calls last_st(dst, at, e, l, v, last_pre(e, l)), dst being the buffer it may write to (the value
 // returned) and last_pre what it reads from the tables, asked for before the stage's own work.
-// Long transforms are scaled up to their largest component once or twice on the way (FftPlan::renorm, early;
-// mid two zeroed words of the block) by 2^shift in all, shift >= 0, set before the last stage: data that
-// gather on one element have nothing to scale up and are left as they are.  Ends with a barrier.
+// Long transforms are scaled up to their largest component once more on the way (FftPlan::renorm,
+// *mid a zeroed word of the block) by 2^shift, shift >= 0, set before the last stage: data that gather on
+// one element have nothing to scale up and are left as they are.  Ends with a barrier.
 template <int LG, bool INV, class TAB, class LD, class COOK, class PRE, class ST>
 __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *tw, longlong2 *to, longlong2 *alt,
                                                 unsigned odd, LD &&first_ld, COOK &&cook, PRE &&last_pre, ST &&last_st, unsigned *mid, int &shift) {
-    const int n = pl.n, last = pl.ns - 1, renorm = pl.renorm, early = pl.early;
-    int up = 0;
+    const int n = pl.n, last = pl.ns - 1, renorm = pl.renorm;
     shift = 0;
     dispatch_stage<LG, INV, true, false, TAB>(n, pl.stage[0], tw, odd, first_ld, cook, nothing_ahead,
                                          [&](int at, int, int, longlong2 v, Nothing) { to[at] = v; });
@@ -109,8 +108,8 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
         to = alt;
         alt = const_cast<longlong2 *>(from);
         if (renorm) {
-            const int sh = i == renorm || i == early ? up : 0;
-            const bool late = i + 1 == renorm, track = late || i + 1 == early;
+            const int sh = i == renorm ? shift : 0;
+            const bool track = i + 1 == renorm;
             unsigned mag = 0;
             dispatch_stage<LG, INV, false, false, TAB>(
                 n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; },
@@ -119,12 +118,9 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
                     to[at] = v;
                     mag |= mag32(v);
                 });
-            if (track) block_or(mag, mid + late);
+            if (track) block_or(mag, mid);
             __syncthreads();
-            if (track) {
-                up = max(0, pl.renorm_bits - 32 - bit_length(mid[late]));
-                shift += up;
-            }
+            if (track) shift = max(0, pl.renorm_bits - 32 - bit_length(*mid));
         } else {
             dispatch_stage<LG, INV, false, false, TAB>(n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; }, as_read, nothing_ahead,
                                                   [&](int at, int, int, longlong2 v, Nothing) { to[at] = v; });
@@ -247,11 +243,11 @@ __device__ __forceinline__ void rows_item(const TestDesc &T, int unit, double2 *
     const bool self = pr.x == pr.y;
     const unsigned odd = parity(pr.x) | parity(pr.y) << 1;  // of the lanes' rows
     int sx, sy;
-    longlong2 *X = rows_forward<TAB>(T, pr, xd, sm, sm + 2 * C, odd, &ctl.top[0], &ctl.mag[0], ctl.mid[0], sx);
+    longlong2 *X = rows_forward<TAB>(T, pr, xd, sm, sm + 2 * C, odd, &ctl.top[0], &ctl.mag[0], &ctl.mid[0], sx);
     longlong2 *other = X == sm ? sm + 2 * C : sm;
     longlong2 *Y = X;
     if constexpr (MUL) {
-        Y = rows_forward<TAB>(T, pr, yd, other, sm + 4 * C, odd, &ctl.top[1], &ctl.mag[1], ctl.mid[1], sy);
+        Y = rows_forward<TAB>(T, pr, yd, other, sm + 4 * C, odd, &ctl.top[1], &ctl.mag[1], &ctl.mid[1], sy);
         other = Y == other ? sm + 4 * C : other;
     } else {
         sy = sx;
@@ -299,7 +295,7 @@ __device__ __forceinline__ void rows_item(const TestDesc &T, int unit, double2 *
             (l ? ob : oa)[e] = v;
             mag |= mag32(v);
         },
-        ctl.mid[2], shift);
+        &ctl.mid[2], shift);
     block_or(mag, &ctl.mag_out);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -539,7 +535,7 @@ __device__ __forceinline__ void col_inverse_item(const TestDesc &T, int g, int s
             big |= mag32(v);
             dst[turned<LG>(r, l)] = v;
         },
-        ctl.mid[0], shift);
+        &ctl.mid[0], shift);
     const bool short_transform = n + shift < 0;  // the last place is above 1: too short for its data
     segment_carries<1 << LG, TAB>(T, g, digits);
     // |digit| >= 2^51 reports 0.5, as does a transform too short for its data
@@ -624,7 +620,7 @@ __device__ __forceinline__ void col_forward_item(const TestDesc &T, int g, doubl
             const longlong2 z = cmul(v, w, half_of(parity(k) ^ ((odd >> l) & 1)));
             xg[e] = make_double2(from_fixed(z.x, ex - up), from_fixed(z.y, ex - up));
         },
-        ctl.mid[0], up);
+        &ctl.mid[0], up);
 }
 
 // One column group of one test: its digits.  Ends with a barrier.
@@ -662,7 +658,7 @@ __device__ __forceinline__ void col_digits_item(const TestDesc &T, int g, const 
             dig[j] = shift_by(scale_round(v.x, o.x, max(0, min(m, 95)), f), max(0, -m));
             dig[j + 1] = shift_by(scale_round(v.y, o.y, max(0, min(m, 95)), f), max(0, -m));
         },
-        ctl.mid[0], shift);
+        &ctl.mid[0], shift);
 }
 
 }  // namespace kg

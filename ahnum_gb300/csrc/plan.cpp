@@ -272,19 +272,18 @@ bool make_fft_plan(int n, FftPlan &pl) {
     // round-off below half of what FP64 had at the same length; longer transforms take the bits
     // back before their last two stages, else the loss would pass FP64's from 2^9 points on.  Data that
     // gather on one element keep the bound itself, components up to 2^62, and are never scaled down.
-    // Scaled up to components below 2^61 (moduli below 2^61.5), the last two stages have to stay below
-    // 2^63: their growth is at most 1 where both are of radix 4, 2.5 else, and 3.5 at 686 = 7 7 7 2 alone,
+    // Scaled up to components below 2^61 (moduli below 2^61.5), the stages left have to stay below
+    // 2^63: their growth is at most 1 where they are of radix 4, 2.5 else, and 3.5 at 686 = 7 7 7 2 alone,
     // which is scaled to 2^60.  The first stage whose output can be looked at is stage 1.
     // A twiddled radix 3 takes more from random data than radix 4 (sqrt(3) / 4 against 1 / 2) and its
-    // butterflies round more, so plans of 6 stages with three odd ones scale up before stage 2 as well.
-    // Largest round-off at 734832 digits (rows of 1512 = 7 3 3 3 2 4) 0.30 without, 0.12 so, FP64 0.23; at
-    // 967680 (1080) 0.18, 0.08 and 0.14.
+    // butterflies round more, so plans of 6 stages with three odd ones scale up before stage 2 instead.
+    // Largest round-off at 734832 digits (rows of 1512 = 7 3 3 3 2 4) 0.30 before the last two, 0.12 so, FP64
+    // 0.23; at 967680 (1080) 0.18, 0.06 and 0.14.  Scaling up at both costs the pass kernels 2 %.
     if (n > 256 && pl.ns >= 4) {
-        pl.renorm = pl.ns - 2;
         const int odd = (int)std::count_if(rad.begin(), rad.end(), [](int p) { return p % 2 && p > 1; });
-        if (odd >= 3 && pl.renorm > 3) pl.early = 2;
+        pl.renorm = odd >= 3 && pl.ns >= 6 ? 2 : pl.ns - 2;
         double tail = 1, peak = 1;
-        for (int i = pl.early ? pl.early : pl.renorm; i < pl.ns; i++) {
+        for (int i = pl.renorm; i < pl.ns; i++) {
             tail *= pl.stage[i].radix > 2 ? pl.stage[i].radix / 4.0 : 2;
             peak = std::max(peak, tail);
         }

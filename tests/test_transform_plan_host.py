@@ -22,8 +22,8 @@ def _growth(i, p):
 def test_plans_of_every_length(lib):
     scaled = []
     for n in _lengths():
-        radix, head, early, renorm, bits = (C.c_int * 8)(), C.c_int(), C.c_int(), C.c_int(), C.c_int()
-        ns = lib.kc_transform_plan(n, radix, C.byref(head), C.byref(early), C.byref(renorm), C.byref(bits))
+        radix, head, renorm, bits = (C.c_int * 8)(), C.c_int(), C.c_int(), C.c_int()
+        ns = lib.kc_transform_plan(n, radix, C.byref(head), C.byref(renorm), C.byref(bits))
         assert 2 <= ns <= 8 and math.prod(radix[:ns]) == n
         # squares of moduli: components of 2^b make a modulus of sqrt(2) 2^b
         at, peak = Fraction(1), Fraction(1)
@@ -32,15 +32,14 @@ def test_plans_of_every_length(lib):
             peak = max(peak, at)
         assert 2 * (peak * Fraction(2) ** (62 - head.value)) ** 2 <= Fraction(2) ** 124, n
         if not renorm.value:
-            assert (n <= 256 or ns < 4) and not early.value
+            assert n <= 256 or ns < 4
             continue
         scaled.append(n)
         # stage 1 is the first whose outputs are looked at, and the last stage does not scale
         assert 2 <= renorm.value <= ns - 2, n
         assert 32 < bits.value <= 61, n
-        assert early.value in (0, 2) and early.value < renorm.value, n
         at, peak = Fraction(1), Fraction(1)
-        for i in range(early.value or renorm.value, ns):  # the second may find nothing to scale up
+        for i in range(renorm.value, ns):
             at *= _growth(i, radix[i])
             peak = max(peak, at)
         assert 2 * (peak * Fraction(2) ** bits.value) ** 2 < Fraction(2) ** 126 * Fraction(99, 100), n
@@ -48,6 +47,6 @@ def test_plans_of_every_length(lib):
 
 
 def test_lengths_without_a_plan(lib):
-    radix, v = (C.c_int * 8)(), [C.c_int() for _ in range(4)]
+    radix, v = (C.c_int * 8)(), [C.c_int() for _ in range(3)]
     for n in (0, 1, 11, 22, 26, 1331):
         assert lib.kc_transform_plan(n, radix, *map(C.byref, v)) == -1
