@@ -415,6 +415,11 @@ kc_engine *kc_engine_create(uint64_t k, uint64_t n, uint32_t L, const uint8_t *b
         d.G = e->G;
         d.rp = P.rp;
         d.cp = P.cp;
+        // narrow digits: the same stages and tables, scaled elsewhere on the way
+        if (*std::max_element(e->lay.bits.begin(), e->lay.bits.end()) <= kNarrowBits) {
+            make_fft_plan((int)P.C, d.rp, true);
+            make_fft_plan((int)P.R, d.cp, true);
+        }
         d.twr = P.twr;
         d.twc = P.twc;
         d.t4 = P.t4;

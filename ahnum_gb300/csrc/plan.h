@@ -33,8 +33,10 @@ bool throughput_group(uint32_t H, unsigned min_bits, unsigned top_digits, uint32
 bool set_shape_override(uint32_t L, uint32_t R);
 // Usable shapes of H = R*C near balance, at most `max`; returns the count.
 int shape_candidates(uint32_t H, uint32_t *R, uint32_t *C, int max);
-// The stages of a length-n transform; false if n has a prime factor above 7.
-bool make_fft_plan(int n, FftPlan &pl);
+// The stages of a length-n transform; false if n has a prime factor above 7.  narrow: of numbers whose
+// digits have no more than kNarrowBits bits.
+bool make_fft_plan(int n, FftPlan &pl, bool narrow = false);
+constexpr unsigned kNarrowBits = 10;
 
 // exp(-2 pi i j / m), j = 0..m-1, times 2^62 in limbs {c1, c0, s1, s0} (FftStage)
 std::vector<int4> roots_neg(uint32_t m);

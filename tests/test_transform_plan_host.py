@@ -4,6 +4,8 @@ import ctypes as C
 import math
 from fractions import Fraction
 
+import pytest
+
 
 def _lengths():
     def smooth(n):
@@ -19,11 +21,12 @@ def _growth(i, p):
     return Fraction(p, 4) if i and p > 2 else Fraction(p)
 
 
-def test_plans_of_every_length(lib):
+@pytest.mark.parametrize("narrow", [0, 1])
+def test_plans_of_every_length(lib, narrow):
     scaled = []
     for n in _lengths():
         radix, head, renorm, bits = (C.c_int * 8)(), C.c_int(), C.c_int(), C.c_int()
-        ns = lib.kc_transform_plan(n, radix, C.byref(head), C.byref(renorm), C.byref(bits))
+        ns = lib.kc_transform_plan(n, narrow, radix, C.byref(head), C.byref(renorm), C.byref(bits))
         assert 2 <= ns <= 8 and math.prod(radix[:ns]) == n
         # squares of moduli: components of 2^b make a modulus of sqrt(2) 2^b
         at, peak = Fraction(1), Fraction(1)
@@ -32,7 +35,7 @@ def test_plans_of_every_length(lib):
             peak = max(peak, at)
         assert 2 * (peak * Fraction(2) ** (62 - head.value)) ** 2 <= Fraction(2) ** 124, n
         if not renorm.value:
-            assert n <= 256 or ns < 4
+            assert n <= 256 and not narrow or ns < 4
             continue
         scaled.append(n)
         # stage 1 is the first whose outputs are looked at, and the last stage does not scale
@@ -49,4 +52,4 @@ def test_plans_of_every_length(lib):
 def test_lengths_without_a_plan(lib):
     radix, v = (C.c_int * 8)(), [C.c_int() for _ in range(3)]
     for n in (0, 1, 11, 22, 26, 1331):
-        assert lib.kc_transform_plan(n, radix, *map(C.byref, v)) == -1
+        assert lib.kc_transform_plan(n, 0, radix, *map(C.byref, v)) == -1
