@@ -1,5 +1,5 @@
 // The zero test of two numbers, element-wise operations, and the FP64 probes (see device.h for the
-// data layout; the pass kernels are in rows.cu and columns.cu).
+// data layout; the pass kernels are in rows.cu, columns_inverse.cu and columns_forward.cu).
 #include <cuda_runtime.h>
 
 #include <mutex>
