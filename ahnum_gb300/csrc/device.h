@@ -38,8 +38,7 @@ struct FftPlan {
     int ns = 0;        // 2 or more
     int headroom = 0;  // bits the modulus of the input stays below 2^62
     int scale = 0;     // the transform leaves a factor 2^-scale
-    int renorm = 0;    // the stage before which the values are scaled up again (0: none)
-    int renorm_bits = 0;  // then to components below 2^renorm_bits
+    int renorm = 0;    // the stage before which the values are scaled up to components below 2^61 (0: none)
     FftStage stage[kMaxStages] = {};
 };
 

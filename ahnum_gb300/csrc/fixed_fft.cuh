@@ -12,7 +12,7 @@
 // Representation.  A transform holds complex numbers as two int64.  Its input is scaled so that
 // every modulus is at most 2^62 / growth (FftPlan::headroom), where growth bounds what the stages
 // can add up, so no data can overflow; what is scaled up again on the way stays below 2^63 by the
-// growth of the stages that are left (FftPlan::renorm_bits).  Twiddles are scaled by 2^62 and stored as two signed
+// growth of the stages that are left (FftPlan::renorm).  Twiddles are scaled by 2^62 and stored as two signed
 // 32-bit limbs a component; a twiddle product keeps the upper 64 bits of 128, so it divides by
 // 4, which is the growth of a radix-4 butterfly: twiddled radix-4 stages keep the bound, and the
 // values lose half a bit a level against the 62 they start from, as random data grow by sqrt(n)

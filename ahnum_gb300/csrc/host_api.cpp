@@ -46,13 +46,12 @@ int kc_carry_digits(uint64_t k, uint64_t n, uint32_t L, int64_t *digits) {
     return 0;
 }
 
-int kc_transform_plan(int n, int narrow, int *radix, int *headroom, int *renorm, int *renorm_bits) {
+int kc_transform_plan(int n, int narrow, int *radix, int *headroom, int *renorm) {
     kg::FftPlan pl;
     if (!kg::make_fft_plan(n, pl, narrow != 0)) return -1;
     for (int i = 0; i < pl.ns; i++) radix[i] = pl.stage[i].radix;
     *headroom = pl.headroom;
     *renorm = pl.renorm;
-    *renorm_bits = pl.renorm_bits;
     return pl.ns;
 }
 

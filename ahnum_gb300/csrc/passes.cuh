@@ -120,7 +120,7 @@ __device__ __forceinline__ longlong2 *transform(const FftPlan &pl, const int4 *t
                 });
             if (track) block_or(mag, mid);
             __syncthreads();
-            if (track) shift = max(0, pl.renorm_bits - 32 - bit_length(*mid));
+            if (track) shift = max(0, 29 - bit_length(*mid));  // components below 2^61
         } else {
             dispatch_stage<LG, INV, false, false, TAB>(n, pl.stage[i], tw, odd, [&](int at, int, int) { return from[at]; }, as_read, nothing_ahead,
                                                   [&](int at, int, int, longlong2 v, Nothing) { to[at] = v; });

@@ -272,9 +272,9 @@ bool make_fft_plan(int n, FftPlan &pl, bool narrow) {
     // round-off below half of what FP64 had at the same length; longer transforms take the bits
     // back before their last two stages, else the loss would pass FP64's from 2^9 points on.  Data that
     // gather on one element keep the bound itself, components up to 2^62, and are never scaled down.
-    // Scaled up to components below 2^61 (moduli below 2^61.5), the stages left have to stay below
-    // 2^63: their growth is at most 1 where they are of radix 4, 2.5 else, and 3.5 at 686 = 7 7 7 2 alone,
-    // which is scaled to 2^60.  The first stage whose output can be looked at is stage 1.
+    // Scaled up to components below 2^61 (moduli below 2^61.5), the stages left have to stay below 2^63.
+    // Their growth is at most 1 where they are of radix 4 and 2.5 else, but for 686 = 7 7 7 2 (3.5), which is
+    // not scaled up.  The first stage whose output can be looked at is stage 1.
     // A twiddled radix 3 takes more from random data than radix 4 (sqrt(3) / 4 against 1 / 2) and its
     // butterflies round more, so plans of 6 stages with three odd ones scale up before stage 2 instead.
     // Largest round-off at 734832 digits (rows of 1512 = 7 3 3 3 2 4) 0.30 before the last two, 0.12 so, FP64
@@ -285,14 +285,17 @@ bool make_fft_plan(int n, FftPlan &pl, bool narrow) {
     // 4.2 bits 0.50 without, 0.18 so, FP64 0.35.
     if ((narrow || n > 256) && pl.ns >= 4) {
         const int odd = (int)std::count_if(rad.begin(), rad.end(), [](int p) { return p % 2 && p > 1; });
-        pl.renorm = narrow || (odd >= 3 && pl.ns >= 6) ? 2 : pl.ns - 2;
-        double tail = 1, peak = 1;
-        for (int i = pl.renorm; i < pl.ns; i++) {
-            tail *= pl.stage[i].radix > 2 ? pl.stage[i].radix / 4.0 : 2;
-            peak = std::max(peak, tail);
-        }
-        pl.renorm_bits = (int)std::floor(62.9 - 0.5 - std::log2(peak));
-        pl.renorm_bits = std::min(pl.renorm_bits, 61);
+        const auto peak = [&](int from) {  // growth of the stages from `from` on
+            double growth = 1, most = 1;
+            for (int i = from; i < pl.ns; i++) {
+                growth *= pl.stage[i].radix > 2 ? pl.stage[i].radix / 4.0 : 2;
+                most = std::max(most, growth);
+            }
+            return most;
+        };
+        constexpr double kMost = 2.6;  // 2^61.5 times that is 0.92 2^63
+        if ((narrow || (odd >= 3 && pl.ns >= 6)) && peak(2) <= kMost) pl.renorm = 2;
+        else if (peak(pl.ns - 2) <= kMost) pl.renorm = pl.ns - 2;
     }
     return true;
 }

@@ -179,7 +179,7 @@ PROTOTYPES = {
     "kc_digits_to_limbs": (C.c_int, [C.c_uint64, C.c_uint64, C.c_uint32, i64p, u64p]),
     "kc_limbs_to_digits": (C.c_int, [C.c_uint64, C.c_uint64, C.c_uint32, u64p, i64p]),
     "kc_carry_digits": (C.c_int, [C.c_uint64, C.c_uint64, C.c_uint32, i64p]),
-    "kc_transform_plan": (C.c_int, [C.c_int, C.c_int] + 4 * [C.POINTER(C.c_int)]),
+    "kc_transform_plan": (C.c_int, [C.c_int, C.c_int] + 3 * [C.POINTER(C.c_int)]),
     "kc_choose_fft_len": (C.c_uint32, [C.c_uint64, C.c_uint64]),
     # the integer-NTT engine (include/kite_ntt.h)
     "kn_engine_new": (vp, [C.c_uint64, C.c_uint64, C.c_int]),

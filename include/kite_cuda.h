@@ -256,11 +256,11 @@ int kc_digits_to_limbs(uint64_t k, uint64_t n, uint32_t L, const int64_t *digits
 int kc_limbs_to_digits(uint64_t k, uint64_t n, uint32_t L, const uint64_t *limbs, int64_t *digits);
 int kc_carry_digits(uint64_t k, uint64_t n, uint32_t L, int64_t *digits);
 /* The plan of a row's or column's transform of n points (no counterpart in the reference), for numbers
- * of digits of at most 10 bits (narrow) or others: the stages'
- * radices into radix[8], the bits that the moduli of its input stay below 2^62, the stage before which
- * the values are scaled up once more (0: none), to components below 2^*renorm_bits.  Returns the number
- * of stages, or -1 if n has none (a prime factor above 7). */
-int kc_transform_plan(int n, int narrow, int *radix, int *headroom, int *renorm, int *renorm_bits);
+ * of digits of at most 10 bits (narrow) or others: the stages' radices into radix[8], the bits that the
+ * moduli of its input stay below 2^62, and the stage before which the values are scaled up once more (0:
+ * none), to components below 2^61.  Returns the number of stages, or -1 if n has none (a prime factor
+ * above 7). */
+int kc_transform_plan(int n, int narrow, int *radix, int *headroom, int *renorm);
 /* FFT length the engine picks for (k, n) (src/ctx.c:107-141), 0 if none. */
 uint32_t kc_choose_fft_len(uint64_t k, uint64_t n);
 
