@@ -277,12 +277,12 @@ bool make_fft_plan(int n, FftPlan &pl, bool narrow) {
     // not scaled up.  The first stage whose output can be looked at is stage 1.
     // A twiddled radix 3 takes more from random data than radix 4 (sqrt(3) / 4 against 1 / 2) and its
     // butterflies round more, so plans of 6 stages with three odd ones scale up before stage 2 instead.
-    // Largest round-off at 734832 digits (rows of 1512 = 7 3 3 3 2 4) 0.30 before the last two, 0.12 so, FP64
-    // 0.23; at 967680 (1080) 0.18, 0.06 and 0.14.  Scaling up at both costs the pass kernels 2 %.
+    // Largest round-off at 734832 digits (rows of 1512 = 7 3 3 3 2 4) 0.30 before the last two, 0.14 so, FP64
+    // 0.23; at 967680 (1080) 0.18, 0.07 and 0.14.  Scaling up at both costs the pass kernels 2 %.
     // Balanced digits lie half a unit below zero on average.  Of narrow ones that is a spectral line, 30 or 40
     // times the others at 250000 digits of 4 bits, and its square takes their bits until the stages have
     // spread it: their transforms, short ones too, scale up early.  Largest round-off at 373248 digits of
-    // 4.2 bits 0.50 without, 0.18 so, FP64 0.35.
+    // 4.2 bits 0.50 without, 0.16 so, FP64 0.35.
     if ((narrow || n > 256) && pl.ns >= 4) {
         const int odd = (int)std::count_if(rad.begin(), rad.end(), [](int p) { return p % 2 && p > 1; });
         const auto peak = [&](int from) {  // growth of the stages from `from` on
